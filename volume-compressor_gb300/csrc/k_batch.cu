@@ -10,6 +10,7 @@
 #include "idct_tile.cuh"
 #include "imma.cuh"
 #include "kernels.cuh"
+#include "rc_lanes.cuh"
 #include "rangecoder.cuh"
 
 namespace vcg {
@@ -138,16 +139,14 @@ __global__ void k_ua_scatter(BatchJob J) {
     }
 }
 
-constexpr int kBatchLaneThreads = 64;
-
-__global__ void __launch_bounds__(kBatchLaneThreads) k_rc_batch_lanes(BatchJob J) {
+__global__ void __launch_bounds__(kLaneThreads) k_rc_batch_lanes(BatchJob J) {
     __shared__ uint32_t bstart[10];   // the band table and a copy of its end (RcLane)
-    __shared__ uint32_t S[12 * kBatchLaneThreads];
+    __shared__ uint32_t S[kLaneWarps][kLaneRows * 32];
     if (threadIdx.x < 10) bstart[threadIdx.x] = J.band_start[threadIdx.x < 9 ? threadIdx.x : 8];
     __syncthreads();
     const uint32_t n_present = J.sort_ctl[kSortBuckets];   // 0 when the scalar kernel decodes this batch
-    if ((uint64_t)blockIdx.x * kBatchLaneThreads >= n_present) return;   // whole CTA idle
-    const uint32_t i = blockIdx.x * kBatchLaneThreads + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t i = 32u * lane_warp_rank(J.sms) + lane;
     const bool active = i < n_present;
     uint32_t u = 0, cap = 0;
     vcd_atom e = {};
@@ -159,13 +158,10 @@ __global__ void __launch_bounds__(kBatchLaneThreads) k_rc_batch_lanes(BatchJob J
         if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
         dst = J.ent + J.ent_off[u];
     }
-    uint32_t *Sl = S + threadIdx.x;
+    if (!__any_sync(0xFFFFFFFFu, active)) return;   // (the graph's grid serves any batch up to its capacity)
     RcLane L;
-    L.init(J.arc + e.off + 1, e.len - 1u, active, bstart, Sl, kBatchLaneThreads, dst, cap);
-    while (__any_sync(0xFFFFFFFFu, L.c != kLaneDone)) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) L.step(bstart, Sl, kBatchLaneThreads);
-    }
+    L.init(J.arc + e.off + 1, e.len - 1u, active, bstart, &S[threadIdx.x >> 5][lane], 32, dst, cap);
+    decode_lanes(L, e.len, bstart);
     if (!active) return;
     const uint32_t cnt = L.n > cap ? cap : L.n;
     J.cnt[u] = cnt | (L.n > cap ? kEntOverflow : 0u) | (L.bad ? kEntBad : 0u);
@@ -419,8 +415,7 @@ static void launch_rc(const BatchJob &J, int num_sms, uint32_t max_ua, cudaStrea
         k_ua_hist<<<sg, 256, 0, s>>>(J);
         launch_len_scan(J.sort_ctl, s);
         k_ua_scatter<<<sg, 256, 0, s>>>(J);
-        const uint64_t lg = ((uint64_t)max_ua + kBatchLaneThreads - 1) / kBatchLaneThreads;
-        k_rc_batch_lanes<<<(unsigned)(lg < 1 ? 1 : lg), kBatchLaneThreads, 0, s>>>(J);
+        k_rc_batch_lanes<<<lane_grid(max_ua < 1 ? 1 : max_ua, (uint32_t)num_sms), kLaneThreads, 0, s>>>(J);
     }
     // capacity within the latency decoder's range: stage the streams (one CTA
     // per SM at most, with a warp per atom)

@@ -20,6 +20,7 @@
 #include "kernels.cuh"
 #include "idct_tile.cuh"
 #include "rangecoder.cuh"
+#include "rc_lanes.cuh"
 
 namespace vcg {
 
@@ -240,15 +241,13 @@ __global__ void k_len_scatter(DecodeJob J) {
 
 static_assert(kSortBuckets == 4 * 1024, "k_len_scan: 1024 threads x 4 counters");
 
-constexpr int kLaneThreads = 64;   // 2 warps per CTA
-constexpr int kLaneUnroll = 8;     // steps between warp votes
-
-__global__ void __launch_bounds__(kLaneThreads) k_rc_lanes(DecodeJob J) {
+__global__ void __launch_bounds__(kLaneThreads) k_rc_lanes(DecodeJob J, uint32_t sms) {
     __shared__ uint32_t bstart[10];   // the band table and a copy of its end (RcLane)
-    __shared__ uint32_t S[12 * kLaneThreads];   // magnitude contexts, lane-interleaved
+    __shared__ uint32_t S[kLaneWarps][kLaneRows * 32];
     if (threadIdx.x < 10) bstart[threadIdx.x] = J.band_start[threadIdx.x < 9 ? threadIdx.x : 8];
     __syncthreads();
-    const uint64_t i = (uint64_t)blockIdx.x * kLaneThreads + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t i = 32ull * lane_warp_rank(sms) + lane;
     const bool active = i < J.sort_ctl[kSortBuckets];
     uint64_t t = 0;
     vcd_atom e = {};
@@ -263,13 +262,9 @@ __global__ void __launch_bounds__(kLaneThreads) k_rc_lanes(DecodeJob J) {
         if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
         dst = J.ent + J.ent_off[t];
     }
-    uint32_t *Sl = S + threadIdx.x;
     RcLane L;
-    L.init(J.arc + e.off + 1, e.len - 1u, active, bstart, Sl, kLaneThreads, dst, cap);
-    while (__any_sync(0xFFFFFFFFu, L.c != kLaneDone)) {
-#pragma unroll
-        for (int k = 0; k < kLaneUnroll; ++k) L.step(bstart, Sl, kLaneThreads);
-    }
+    L.init(J.arc + e.off + 1, e.len - 1u, active, bstart, &S[threadIdx.x >> 5][lane], 32, dst, cap);
+    decode_lanes(L, e.len, bstart);
     if (!active) return;
     const uint32_t n = L.n > cap ? cap : L.n;
     J.cnt[t] = n | (L.n > cap ? kEntOverflow : 0u) | (L.bad ? kEntBad : 0u);
@@ -355,8 +350,8 @@ static void launch_rc(const DecodeJob &J, int num_sms, cudaStream_t s, const Sta
             Jl.order = J.order + ns;
             Jl.sort_ctl = J.sort_ctl + 2;   // Jl.sort_ctl[kSortBuckets]: the per-lane count
         }
-        const uint64_t lane_blocks = (J.n_atoms - ns + kLaneThreads - 1) / kLaneThreads;
-        if (lane_blocks) k_rc_lanes<<<(unsigned)lane_blocks, kLaneThreads, 0, s>>>(Jl);   // (0: every atom solo)
+        const unsigned lane_blocks = lane_grid(J.n_atoms - ns, (uint32_t)num_sms);
+        if (lane_blocks) k_rc_lanes<<<lane_blocks, kLaneThreads, 0, s>>>(Jl, (uint32_t)num_sms);   // (0: every atom solo)
         if (ns) cudaStreamWaitEvent(s, ev->join, 0);
         return;
     }
@@ -446,7 +441,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_decode_fused(DecodeJob J, 
                                                                     uint32_t *fail) {
     extern __shared__ int32_t T[];   // transform tile
     __shared__ uint32_t bstart[10];   // the band table and a copy of its end (RcLane)
-    __shared__ uint32_t S[12 * kFusedRcThreads];
+    __shared__ uint32_t S[kFusedRcThreads / 32][kLaneRows * 32];
     __shared__ int32_t dqs[VCD_NCLASS], dqb[VCD_NCLASS];
     __shared__ uint32_t alt[1024];
     __shared__ uint32_t q_tail;   // slots of this CTA's queue handed out
@@ -489,7 +484,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_decode_fused(DecodeJob J, 
             }
             return;
         }
-        uint32_t *Sl = S + tid;
+        uint32_t *Sl = &S[tid >> 5][tid & 31];
         uint32_t k = 1u + (uint32_t)tid, t = 0, cap = 0;   // the CTA's entries after its head
         bool have = false;
         RcLane L;
@@ -506,12 +501,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_decode_fused(DecodeJob J, 
                 if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
                 dst = J.ent + J.ent_off[t];
             }
-            L.init(J.arc + e.off + 1, e.len - 1u, have, bstart, Sl, kFusedRcThreads, dst, cap);
+            L.init(J.arc + e.off + 1, e.len - 1u, have, bstart, Sl, 32, dst, cap);
         };
         start();
         while (__any_sync(0xFFFFFFFFu, have)) {
-#pragma unroll
-            for (int s = 0; s < kLaneUnroll; ++s) L.step(bstart, Sl, kFusedRcThreads);
+            L.step(bstart, Sl, 32);
             if (have && L.c == kLaneDone) {   // finished: counts, then publish the atom
                 const uint32_t m = L.n > cap ? cap : L.n;
                 J.cnt[t] = m | (L.n > cap ? kEntOverflow : 0u) | (L.bad ? kEntBad : 0u);

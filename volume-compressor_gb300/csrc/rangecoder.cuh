@@ -279,66 +279,132 @@ __device__ __forceinline__ int rc_decode_levels_warp(const uint8_t *src, uint32_
 }
 
 // ---------------------------------------------------------------- per-lane decoder
-// Each lane of a warp decodes its own atom and every step is one binary
-// decision of that atom, whatever its kind: the lanes of a warp are at
-// different points of their streams, and no lane waits for another (unlike the
-// lockstep decoder, whose warps run every magnitude step as long as any lane
-// needs it). The decision kind is the lane's state:
-//   0        significance bit of scan position p (band context, a register)
-//   1..12    unary magnitude step c - 1 (context mag[c - 1] in shared memory)
-//   13       escape: exponential-Golomb prefix of ones (bypass)
-//   14       bypass run: the escape suffix bits, then the sign bit
-//   15       done
-// (src/vc/vc.c:491-506, 545-560). A bypass bit is the adaptive split with
-// probability 2048 and no adaptation, except that the range becomes the half
-// for both bit values (src/vc/vc.c:431-441). The magnitude context of the next
-// step is loaded from shared memory one step ahead. Stream bytes are fetched
-// one at a time, one byte ahead of the renormalisation that consumes them;
-// bytes past the end read as zero. Probabilities are kept unscaled (12 bits).
-__device__ __forceinline__ uint32_t ld_u8_if(bool on, const uint8_t *ptr, uint32_t old) {
-#ifdef __CUDA_ARCH__
-    uint32_t v = old;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.u8 %0, [%1];\n\t}"
-                 : "+r"(v) : "l"(ptr), "r"((uint32_t)on));
-    return v;
-#else
-    return on ? *ptr : old;
-#endif
-}
-__device__ __forceinline__ void st_u32_if(bool on, uint32_t *ptr, uint32_t v) {
-#ifdef __CUDA_ARCH__
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.u32 [%0], %1;\n\t}"
-                 :: "l"(ptr), "r"(v), "r"((uint32_t)on) : "memory");
-#else
-    if (on) *ptr = v;
-#endif
-}
-
+// Each lane of a warp decodes its own atom (src/vc/vc.c:491-506, 545-560) in
+// rounds that all lanes take together. A round is: up to kZ zeros of the
+// significance run at once (optional), four adaptive decisions of whatever
+// context the lane is at (the significance of the next position, or the next
+// step of the unary magnitude), a few escape bits if a lane of the warp is in an
+// escape, and the sign bit with the store of a finished level. A lane whose
+// state has no part in a piece of the round sits it out.
+//
+// What bounds it on GB300 is the integer ALU (16 lanes per SM sub-partition: an
+// instruction takes it two cycles) and the chain of one decision, so the round
+// is written for few ALU instructions and short dependences (measured there: a
+// multiply high 8.8 cycles, a compare and a select on it 8, but a compare and
+// an instruction guarded by it 18, a branch 18-23): selects instead of guards
+// wherever the next decision waits for the result, no branch inside a round.
+// * A zero only shrinks the range, so a run of zeros without renormalisation
+//   is a chain of multiplies whose splits all exceed max(code, 2^24 - 1); the
+//   first one that does not ends it, and the lane goes on decision by decision.
+// * Four decisions take at most four stream bytes: they come from one register
+//   (a byte permute with a running selector); the next words of the stream are
+//   loaded a round or more before they are needed.
+// * The state is the shared-memory address of the context in use, so the step
+//   after a one is an addition, and the context after it is always prefetched.
+// * What a lane may meet near the end of its stream or of a band (bytes past
+//   the end read as zero, a fresh significance context, the EOB) is left to a
+//   second form of the round (END), taken when a lane of the warp is near one.
+// Measured (1,024 atoms of the 1024^3 benchmark volume, replicated to 32,768
+// in warps of 32 different ones; before: one decision a step, whatever its
+// kind, 82 instructions): 8.62 -> 4.4 ms at target 10 (kZ = 0), 6.15 -> 2.85 at
+// 20 and 1.30 -> 0.56 at 100 (kZ = 6), with the warps placed as in rc_lanes.cuh.
 constexpr uint32_t kLaneDone = 15u;
+constexpr uint32_t kLaneRows = 17u;          // shared-memory rows of a warp: 13 contexts, and rows only prefetched
+constexpr uint32_t kLaneRow = 128u;          // bytes of a row: a word per lane
+constexpr int kEscBits = 4;                  // escape bits a round takes
+constexpr uint32_t kLaneSel = 0x2107u;       // permute selector: code << 8 | first byte of the window
+
+#ifdef __CUDA_ARCH__
+// Operands: %0 range %1 code %2 selector %3 probability in use %4 probability
+// after a one %5 context address %6 positions left in the band %7 address of a
+// finished magnitude (0: none) %8 stream window %9 address of the lane's row 0
+#define VC_LANE_Z(T0, T1)                                                                                            \
+    "sub.u32 u, 4096, pz;\n\tshl.b32 v, pz, 20;\n\tmul.hi.u32 " T1 ", " T0 ", v;\n\tshr.u32 u, u, 5;\n\t"            \
+    "add.u32 pz, pz, u;\n\tsetp.gt.and.u32 z, " T1 ", th, s;\n\tselp.u32 %0, " T1 ", %0, z;\n\t"                     \
+    "selp.u32 %3, pz, %3, z;\n\t@z sub.u32 %6, %6, 1;\n\t"
+#define VC_LANE_Z6                                                                                                   \
+    "setp.eq.u32 s, %5, %9;\n\tsetp.gt.and.u32 s, %6, 6, s;\n\tmax.u32 th, %1, 0xffffff;\n\tmov.u32 t0, %0;\n\t"     \
+    "mov.u32 pz, %3;\n\t" VC_LANE_Z("t0", "t1") VC_LANE_Z("t1", "t2") VC_LANE_Z("t2", "t3") VC_LANE_Z("t3", "t4")    \
+    VC_LANE_Z("t4", "t5") VC_LANE_Z("t5", "t6")
+// one adaptive decision: a = takes part, b / z = a one / a zero, zs / zl = a
+// zero of the significance / of the magnitude
+#define VC_LANE_U(GO)                                                                                                \
+    "shl.b32 v, %3, 20;\n\tmul.hi.u32 t, %0, v;\n\tld.shared.u32 n2, [%5+256];\n\t"                                  \
+    "sub.u32 u, 4096, %3;\n\tshr.u32 u, u, 5;\n\tadd.u32 p0, %3, u;\n\tshr.u32 u, %3, 5;\n\tsub.u32 p1, %3, u;\n\t"  \
+    "setp.ge.and.u32 b|z, %1, t, a;\n\tselp.u32 tz, t, %0, a;\n\tsub.u32 u, %0, t;\n\tsub.u32 v, %1, t;\n\t"         \
+    "selp.u32 %0, u, tz, b;\n\tselp.u32 %1, v, %1, b;\n\t"                                                           \
+    "setp.lt.u32 q, %0, 0x1000000;\n\tshl.b32 u, %0, 8;\n\tprmt.b32 v, %1, %8, %2;\n\tselp.u32 %0, u, %0, q;\n\t"    \
+    "selp.u32 %1, v, %1, q;\n\t@q sub.u32 %2, %2, 1;\n\t"                                                            \
+    "selp.u32 u, p1, p0, b;\n\t@a st.shared.u32 [%5], u;\n\tselp.u32 %3, %4, p0, b;\n\tselp.u32 %4, n2, %4, b;\n\t"  \
+    "setp.eq.and.u32 zs|zl, %5, %9, z;\n\t@zl mov.u32 %7, %5;\n\t@zs sub.u32 %6, %6, 1;\n\t"                         \
+    "add.u32 u, %5, 128;\n\tselp.u32 %5, u, %5, b;\n\tsetp.ne.and.u32 a, %5, l, b;\n\t" GO
+#define VC_LANE_GO "or.pred a, a, zs;\n\t"
+#define VC_LANE_GO_END "setp.ne.and.u32 s, %6, 0, zs;\n\tor.pred a, a, s;\n\t"
+#define VC_LANE_BLOCK(ZEROS, GO)                                                                                     \
+    asm volatile("{\n\t.reg .pred a,b,z,s,q,zs,zl;\n\t.reg .u32 t,u,v,l,th,pz,p0,p1,n2,tz,t0,t1,t2,t3,t4,t5,t6;\n\t" \
+                 "add.u32 l, %9, 1664;\n\t" ZEROS                                                                    \
+                 "setp.lt.u32 a, %5, l;\n\tsetp.ne.and.u32 a, %6, 0, a;\n\t"                                         \
+                 VC_LANE_U(GO) VC_LANE_U(GO) VC_LANE_U(GO) VC_LANE_U(GO) "}"                                         \
+                 : "+r"(range), "+r"(code), "+r"(sel), "+r"(pr), "+r"(nx), "+r"(sa), "+r"(left), "+r"(m)             \
+                 : "r"(w), "r"(base)                                                                                 \
+                 : "memory")
+#endif
 
 struct RcLane {
-    const uint8_t *src;
-    uint32_t pos, len;     // next byte to fetch; stream length
-    uint32_t nxt;          // the byte at pos (0 past the end)
+    const uint8_t *wp, *end;      // next stream word to load; end of the stream
+    uint32_t a0, a1, a2, pf, o;   // stream words from the one in use, the one loaded last (raw), bits of a0 used
     uint32_t code, range;
-    uint32_t c, r, m;      // state; escape / run count; magnitude so far
-    uint32_t p, eob, bend, bi;   // scan position, EOB, end of the current band, band
-    uint32_t sigp, magp;   // context of the current band; magnitude context of the next step
-    uint32_t *dst;         // coefficient list (scan position | level << 16)
-    uint32_t n, cap, bad;  // entries decoded (all, also past cap); list capacity; malformed
+    uint32_t pr, nx;              // probability of the context in use, and of the one after a one
+    uint32_t base, sa;            // row 0 of the lane (significance), row of the context in use (kEsc, kDone)
+    uint32_t left;                // positions from the current one to the end of its band or the EOB
+    uint32_t m;                   // row address of a finished magnitude whose sign is due, else 0
+    uint32_t x, mag;              // escape: ones of the prefix, then suffix bits due (bit 31 set); value so far
+    uint32_t eob, bend, bi;       // EOB, end of the current band (EOB at most), band
+    uint32_t *dst;                // coefficient list (scan position | level << 16)
+    uint32_t n, cap, bad;         // entries decoded (all, also past cap); list capacity; malformed
+    uint32_t c;                   // kLaneDone once the atom is decoded
+    static constexpr uint32_t kEsc = 13u * kLaneRow, kDone = 14u * kLaneRow;
+#ifndef __CUDA_ARCH__
+    uint32_t sig0;                // (host: row 0; rows 1-12 are S[0], S[st], ...)
+    uint32_t *hS, hst;
+    uint32_t row_ld(uint32_t a) const {
+        const uint32_t r = (a - base) / kLaneRow;
+        return r == 0 ? sig0 : r <= 12u ? hS[(r - 1u) * hst] : 2048u;
+    }
+    void row_st(uint32_t a, uint32_t v) {
+        const uint32_t r = (a - base) / kLaneRow;
+        if (r == 0) sig0 = v;
+        else if (r <= 12u) hS[(r - 1u) * hst] = v;
+    }
+#endif
 
-    // bstart: the 9-entry band table followed by a copy of its last entry (a
-    // lane that ends at the last band's end loads the entry after it).
-    // S: this lane's 12 magnitude contexts at S[0], S[st], ..., S[11 * st]
+    __device__ __forceinline__ static uint32_t be(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
+    __device__ __forceinline__ static uint32_t stream_mask(int rem) {   // of a word with rem stream bytes from its first on
+        return rem >= 4 ? 0xFFFFFFFFu : rem <= 0 ? 0u : 0xFFFFFFFFu << (8 * (4 - rem));
+    }
+    __device__ __forceinline__ uint32_t load_word() {   // raw word at wp if it holds a stream byte
+        const uint32_t v = (int)(end - wp) > 0 ? __ldg(reinterpret_cast<const uint32_t *>(wp)) : 0u;
+        wp += 4;
+        return v;
+    }
+    __device__ __forceinline__ void finish() {   // nothing of the lane is near an end any more
+        sa = base + kDone;
+        left = 0x40000000u;
+        end = wp + 64;
+        c = kLaneDone;
+    }
+
+    // bstart: the 9-entry band table followed by a copy of its last entry.
+    // S: device: the lane's word of the warp's kLaneRows rows, which are st = 32
+    // words apart (row 0 the significance context, row c the one of magnitude
+    // step c); host: 12 words st apart
     __device__ __forceinline__ void init(const uint8_t *s, uint32_t l, bool active, const uint32_t *bstart,
                                          uint32_t *S, uint32_t st, uint32_t *d, uint32_t cp) {
-        src = s;
-        len = active ? l : 0u;
-        uint32_t cd = 0;
+        const uint32_t len = active ? l : 0u;
+        end = s + len;
+        uint32_t cd = 0, at = 5;
 #pragma unroll
-        for (uint32_t i = 0; i < 5; ++i) cd = (cd << 8) | (i < len ? (uint32_t)__ldg(src + i) : 0u);
-        pos = 5;
-        nxt = 5 < len ? __ldg(src + 5) : 0u;
+        for (uint32_t i = 0; i < 5; ++i) cd = (cd << 8) | (i < len ? (uint32_t)__ldg(s + i) : 0u);
         uint32_t rg = 0xFFFFFFFFu, e = 0;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {   // 16-bit EOB in bypass bits (src/vc/vc.c:520-525)
@@ -348,80 +414,240 @@ struct RcLane {
             e = (e << 1) | (b ? 1u : 0u);
             if (rg < kTop) {
                 rg <<= 8;
-                cd = (cd << 8) | nxt;
-                ++pos;
-                nxt = pos < len ? __ldg(src + pos) : 0u;
+                cd = (cd << 8) | (at < len ? (uint32_t)__ldg(s + at) : 0u);
+                ++at;
             }
         }
         if (e > 32768u) e = 32768u;   // src/vc/vc.c:549
         code = cd;
         range = rg;
         eob = e;
-        p = 0;
+        const uint32_t mis = (uint32_t)((uintptr_t)(s + at) & 3u);
+        wp = s + at - mis;
+        o = 8u * mis;
+        const int rem = (int)(end - wp);
+        a0 = be(load_word()) & stream_mask(rem);
+        a1 = be(load_word()) & stream_mask(rem - 4);
+        a2 = be(load_word()) & stream_mask(rem - 8);
+        pf = load_word();
         bi = 0;
-        bend = bstart[1];
-        sigp = 2048u;
-        magp = 2048u;
+        bend = bstart[1] < e ? bstart[1] : e;
+        left = bend;
+#ifdef __CUDA_ARCH__
 #pragma unroll
-        for (int k = 0; k < 12; ++k) S[k * st] = 2048u;
-        c = (active && e) ? 0u : kLaneDone;
-        r = 0;
-        m = 0;
+        for (uint32_t k = 0; k < kLaneRows; ++k) S[k * st] = 2048u;
+        base = (uint32_t)__cvta_generic_to_shared(S);
+#else
+        hS = S;
+        hst = st;
+        sig0 = 2048u;
+        for (uint32_t k = 0; k < 12; ++k) S[k * st] = 2048u;
+        base = kLaneRow;
+#endif
+        pr = nx = 2048u;
+        m = x = mag = 0;
         dst = d;
         n = 0;
         cap = cp;
         bad = 0;
+        c = 0;
+        sa = base;
+        if (!active || !e) {
+            o = 0;
+            finish();
+        }
     }
 
+    // a lane whose next round may meet the end of its band (a round takes at most
+    // kZ + 5 positions), or whose stream word in use is not a0; near_end: or which
+    // may meet the end of its stream in one of two rounds (a word each)
+    template <int kZ>
+    __device__ __forceinline__ bool near_band() const {
+        return left < (uint32_t)(kZ + 6) || o >= 32u;
+    }
+    template <int kZ>
+    __device__ __forceinline__ bool near_end() const {
+        return (int)(end - wp) < 16 || near_band<kZ>();
+    }
+    __device__ __forceinline__ void next_word_end() {
+        a0 = a1;
+        a1 = a2;
+        a2 = be(pf) & stream_mask((int)(end - wp) + 4);
+        pf = load_word();
+        o -= 32u;
+    }
+    __device__ __forceinline__ void renorm(uint32_t w, uint32_t &sel) {
+        const bool q = range < kTop;
+        const uint32_t c1 = __byte_perm(code, w, sel);
+        range = q ? range << 8 : range;
+        code = q ? c1 : code;
+        sel -= q ? 1u : 0u;
+    }
+    __device__ __forceinline__ bool bypass(bool on, uint32_t w, uint32_t &sel) {   // src/vc/vc.c:431-441
+        const uint32_t t = range >> 1;
+        const bool b = on && code >= t;
+        code = b ? code - t : code;
+        range = on ? t : range;
+        renorm(w, sel);
+        return b;
+    }
+
+    // One round of every lane of the warp. END: a lane may be near an end
+    // (near_end<kZ>). ESC: with escape bits.
+    template <int kZ, bool END, bool ESC>
+    __device__ __forceinline__ void round(const uint32_t *bstart) {
+        static_assert(kZ == 0 || kZ == 6, "zeros taken at once");
+        if (END)
+            while (o >= 32u) next_word_end();
+        uint32_t w = __funnelshift_l(a1, a0, o);
+        const uint32_t w1 = __funnelshift_l(a2, a1, o);
+        uint32_t sel = kLaneSel;
+#ifdef __CUDA_ARCH__
+        if (kZ == 0) {
+            if (END) VC_LANE_BLOCK("", VC_LANE_GO_END);
+            else VC_LANE_BLOCK("", VC_LANE_GO);
+        } else {
+            if (END) VC_LANE_BLOCK(VC_LANE_Z6, VC_LANE_GO_END);
+            else VC_LANE_BLOCK(VC_LANE_Z6, VC_LANE_GO);
+        }
+#else
+        if (sa == base && left > (uint32_t)kZ) {
+            const uint32_t th = code > kTop - 1u ? code : kTop - 1u;
+            for (int i = 0; i < kZ; ++i) {
+                const uint32_t t = __umulhi(range, pr << 20);
+                if (t <= th) break;
+                range = t;
+                pr = rc_adapt(pr, false);
+                --left;
+            }
+        }
+        bool go = sa < base + kEsc && left != 0;
+        for (int i = 0; i < 4 && go; ++i) {
+            const uint32_t t = rc_split(range, pr), n2 = row_ld(sa + 2u * kLaneRow);
+            const bool b = code >= t;
+            code = b ? code - t : code;
+            range = b ? range - t : t;
+            row_st(sa, rc_adapt(pr, b));
+            renorm(w, sel);
+            if (b) {
+                pr = nx;
+                nx = n2;
+                sa += kLaneRow;
+                go = sa != base + kEsc;
+            } else if (sa == base) {
+                pr = sig0;
+                --left;
+                go = left != 0;
+            } else {
+                m = sa;
+                go = false;
+            }
+        }
+#endif
+        // bytes taken by the four decisions; the window moves on by them
+        const uint32_t used = 8u * (kLaneSel - sel);
+        w = used == 32u ? w1 : __funnelshift_l(w1, w, used);
+        sel = kLaneSel;
+        if (ESC && __any_sync(0xFFFFFFFFu, sa == base + kEsc)) {   // exponential-Golomb escape: a few bits a round, in selects
+#pragma unroll
+            for (int i = 0; i < kEscBits; ++i) {
+                const bool on = sa == base + kEsc && m == 0 && x != 33u, suffix = (int32_t)x < 0;
+                const bool b = bypass(on, w, sel);
+                const uint32_t xn = suffix ? x - 1u : (b ? x + 1u : x | 0x80000000u);   // prefix ends: its ones are due
+                const uint32_t mn = suffix ? 2u * mag + (b ? 1u : 0u) : 1u;
+                const bool fin = on && xn == 0x80000000u;   // no suffix bit due any more
+                m = fin ? base + ((11u + mn) & 0xFFFFu) * kLaneRow : m;
+                x = on ? (fin ? 0u : xn) : x;
+                mag = on ? mn : mag;
+            }
+            if (x == 33u) {   // a prefix longer than any level needs: malformed
+                bad = 1;
+                finish();
+            }
+        }
+        // sign bit and store of a finished level, then the significance of the next position
+        const uint32_t pos = bend - left;
+#ifdef __CUDA_ARCH__
+        asm volatile(
+            "{\n\t.reg .pred on, b, q, e;\n\t.reg .u32 t, u, v, sg, n1;\n\t.reg .u64 d;\n\t"
+            "ld.shared.u32 sg, [%12];\n\tld.shared.u32 n1, [%12+128];\n\t"
+            "setp.ne.u32 on, %7, 0;\n\tshr.u32 t, %0, 1;\n\tsetp.ge.and.u32 b, %1, t, on;\n\tsub.u32 u, %1, t;\n\t"
+            "selp.u32 %1, u, %1, b;\n\tselp.u32 %0, t, %0, on;\n\tsetp.lt.u32 q, %0, 0x1000000;\n\tshl.b32 u, %0, 8;\n\t"
+            "prmt.b32 v, %1, %9, %2;\n\tselp.u32 %0, u, %0, q;\n\tselp.u32 %1, v, %1, q;\n\t@q sub.u32 %2, %2, 1;\n\t"
+            "sub.u32 u, %7, %12;\n\tshr.u32 u, u, 7;\n\tneg.s32 v, u;\n\tselp.u32 u, v, u, b;\n\t"
+            "prmt.b32 u, %10, u, 0x5410;\n\tsetp.lt.and.u32 e, %8, %11, on;\n\tmad.wide.u32 d, %8, 4, %13;\n\t"
+            "@e st.global.u32 [d], u;\n\t@on add.u32 %8, %8, 1;\n\t@on sub.u32 %6, %6, 1;\n\t"
+            "selp.u32 %5, %12, %5, on;\n\tselp.u32 %3, sg, %3, on;\n\tselp.u32 %4, n1, %4, on;\n\tmov.u32 %7, 0;\n\t}"
+            : "+r"(range), "+r"(code), "+r"(sel), "+r"(pr), "+r"(nx), "+r"(sa), "+r"(left), "+r"(m), "+r"(n)
+            : "r"(w), "r"(pos), "r"(cap), "r"(base), "l"(dst)
+            : "memory");
+#else
+        if (m != 0) {
+            const uint32_t mg = (m - base) / kLaneRow;
+            const bool b = bypass(true, w, sel);
+            if (n < cap) dst[n] = ((b ? 0u - mg : mg) << 16) | pos;
+            ++n;
+            --left;
+            sa = base;
+            pr = sig0;
+            nx = row_ld(base + kLaneRow);
+            m = 0;
+        }
+#endif
+        o += used + 8u * (kLaneSel - sel);
+        if (!END) {
+#ifdef __CUDA_ARCH__
+            asm volatile(
+                "{\n\t.reg .pred c;\n\t.reg .u32 t;\n\tsetp.ge.u32 c, %0, 32;\n\tselp.u32 %1, %2, %1, c;\n\t"
+                "selp.u32 %2, %3, %2, c;\n\tprmt.b32 t, %4, 0, 0x0123;\n\tselp.u32 %3, t, %3, c;\n\t"
+                "@c ld.global.nc.u32 %4, [%5];\n\t@c add.u64 %5, %5, 4;\n\t@c sub.u32 %0, %0, 32;\n\t}"
+                : "+r"(o), "+r"(a0), "+r"(a1), "+r"(a2), "+r"(pf), "+l"(wp));
+#else
+            if (o >= 32u) next_word_end();
+#endif
+        } else {
+            while (o >= 32u) next_word_end();
+            if (left == 0 && sa == base) {   // end of the band: a fresh context, or the EOB
+                if (bend == eob) {
+                    finish();
+                } else {
+                    ++bi;
+                    const uint32_t e = bstart[bi + 1u] < eob ? bstart[bi + 1u] : eob;
+                    left = e - bend;
+                    bend = e;
+                    pr = 2048u;
+#ifndef __CUDA_ARCH__
+                    sig0 = 2048u;
+#endif
+                }
+            }
+        }
+    }
+
+    // rounds of every lane of the warp until some lane has met an end (whole
+    // warp; call until all lanes are done): two at a time, with escape bits in
+    // the second
+    template <int kZ>
+    __device__ __forceinline__ void rounds(const uint32_t *bstart) {
+        while (!__any_sync(0xFFFFFFFFu, near_end<kZ>())) {
+            round<kZ, false, false>(bstart);
+            if (__any_sync(0xFFFFFFFFu, near_band<kZ>())) break;
+            round<kZ, false, true>(bstart);
+        }
+        round<kZ, true, true>(bstart);
+    }
+    // two rounds, or one where a lane may meet an end (whole warp)
     __device__ __forceinline__ void step(const uint32_t *bstart, uint32_t *S, uint32_t st) {
-        const uint32_t s0 = c;
-        const bool isA = s0 < 13u, isPre = s0 == 13u, isRun = s0 == 14u, isSig = s0 == 0u;
-        const uint32_t nmag = S[(s0 < 11u ? s0 : 11u) * st];   // context of step s0 + 1 if this bit is a one
-        const uint32_t pc = isSig ? sigp : magp;
-        const uint32_t pr = isA ? pc : 2048u;
-        const uint32_t r0 = __umulhi(range, pr << 20);
-        const bool b = code >= r0;
-        const uint32_t one = b ? 1u : 0u;
-        code = b ? code - r0 : code;
-        const uint32_t nr = (b && isA) ? range - r0 : r0;
-        const uint32_t pa = rc_adapt(pc, b);
-        if (s0 - 1u < 12u) S[(s0 - 1u) * st] = pa;
-        sigp = isSig ? pa : sigp;
-        magp = nmag;
-        // renormalisation: one byte at most
-        const bool ren = nr < kTop;
-        range = ren ? nr << 8 : nr;
-        code = ren ? (code << 8) | nxt : code;
-        const uint32_t np_ = pos + (ren ? 1u : 0u);
-        pos = np_;
-        nxt = ld_u8_if(ren && np_ < len, src + np_, ren ? 0u : nxt);
-        // the sign bit ends a run of one: emit the level
-        const uint32_t r_ = r, m_ = m;
-        const bool last = isRun && r_ == 1u;
-        const uint32_t sm = b ? 0u - m_ : m_;
-        st_u32_if(last && n < cap, dst + n, (sm << 16) | p);
-        n += last ? 1u : 0u;
-        // next state: a one climbs the ladder (12 -> 13 is the escape); a zero at
-        // significance moves on, a zero on the ladder ends the magnitude (run of
-        // one: the sign); the prefix ends with a zero (run of ones + 1 bits)
-        const uint32_t cA = b ? s0 + 1u : (isSig ? 0u : 14u);
-        const uint32_t cB = isPre ? 14u - one : (last ? 0u : 14u);
-        uint32_t nc = isA ? cA : (s0 == kLaneDone ? kLaneDone : cB);
-        r = isA ? one ^ 1u : (isPre ? r_ + 1u : r_ - 1u);
-        // magnitude: the ladder step that ended it, or 11 + the suffix value
-        m = isA ? s0 : (isPre ? 12u : 2u * m_ + one - 11u);
-        const bool malformed = isPre && b && r_ == 32u;   // a prefix of 33 ones: no level needs it
-        bad |= malformed ? 1u : 0u;
-        const bool adv = (isSig && !b) || last;
-        const uint32_t pn = p + (adv ? 1u : 0u);
-        p = pn;
-        const bool cross = adv && pn == bend;   // next band: fresh context
-        nc = (malformed || (adv && pn == eob)) ? kLaneDone : nc;
-        const uint32_t nbi = bi + (cross ? 1u : 0u);
-        bi = nbi;
-        bend = cross ? bstart[nbi + 1u] : bend;
-        sigp = cross ? 2048u : sigp;
-        c = nc;
+        (void)S;
+        (void)st;
+        if (!__any_sync(0xFFFFFFFFu, near_end<6>())) {
+            round<6, false, false>(bstart);
+            if (!__any_sync(0xFFFFFFFFu, near_band<6>())) {
+                round<6, false, true>(bstart);
+                return;
+            }
+        }
+        round<6, true, true>(bstart);
     }
 };
 
@@ -435,6 +661,16 @@ struct RcLane {
 // atom per SM sub-partition 44 ns per decision against 57 ns. With several
 // warps per sub-partition its extra instructions make it slower, so it serves
 // only the latency-bound case.
+__device__ __forceinline__ uint32_t ld_u8_if(bool on, const uint8_t *ptr, uint32_t old) {
+#ifdef __CUDA_ARCH__
+    uint32_t v = old;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.u8 %0, [%1];\n\t}"
+                 : "+r"(v) : "l"(ptr), "r"((uint32_t)on));
+    return v;
+#else
+    return on ? *ptr : old;
+#endif
+}
 struct RcIn {
     const uint8_t *src;
     uint32_t pos, len, nxt;   // next byte to fetch (nxt: its value, 0 past the end)
