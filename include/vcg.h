@@ -49,20 +49,20 @@ vc_status vcg_set_batch_shape(int rc_scalar_warps, int transform_threads, int tr
 
 // Range-decoder policy of vc_decode_region / vc_decode_lod / vc_decode_atom and
 // the device-output variants (process-wide; results do not depend on it). Up
-// to one atom per SM sub-partition (4 per SM) each atom has a warp running the
-// latency-tuned scalar decoder; up to w warps per sub-partition, one atom per
-// warp with the plain scalar decoder, longest payloads first; above that the
+// to w warps per SM sub-partition (4 per SM) each atom has a warp running a
+// one-atom decoder, longest payloads first above one per sub-partition, on a
+// copy of its stream in shared memory where the streams fit; above that the
 // per-lane decoder (every lane of a warp decodes its own atom, atoms in order
 // of payload length). w = 0: no atom keeps a warp to itself (above one atom
 // per sub-partition the per-lane decoder, below it atoms share warps in
 // lockstep); w < 0 restores the default (8: measured on GB300, the per-lane
-// decoder wins from 3,000-5,000 atoms on, depending on the atoms' sizes).
+// decoder wins from about 4,000 atoms on, depending on the atoms' sizes).
 void vcg_set_rc_scalar_warps(int w);
 // The per-lane decoder's n longest atoms (by payload length) each get a warp of
 // their own running the latency-tuned decoder, on a second stream beside it
 // (process-wide; results do not depend on it). The longest atoms set the
-// per-lane decoder's time, and the latency decoder takes about half the time
-// per decision; whether that shortens the decode depends on which SM
+// per-lane decoder's time, and the latency decoder takes less time per
+// decision; whether that shortens the decode depends on which SM
 // sub-partitions the solo warps land on, which the launch does not control.
 // n = 0 (the default): none; n < 0 restores the default.
 void vcg_set_rc_solo(int n);

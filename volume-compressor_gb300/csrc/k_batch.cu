@@ -34,7 +34,7 @@ __device__ __forceinline__ uint32_t dynamic_smem_bytes() {
 }
 
 __global__ void __launch_bounds__(kRcBatchThreads) k_rc_batch(BatchJob J) {
-    extern __shared__ uint8_t bstage[];
+    extern __shared__ __align__(16) uint8_t bstage[];
     __shared__ uint32_t bstart[9];
     if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
     __syncthreads();
@@ -61,24 +61,8 @@ __global__ void __launch_bounds__(kRcBatchThreads) k_rc_batch(BatchJob J) {
         if (staged) {
             __syncwarp();   // lane 0 is done with the slice (its previous atom)
             const uint32_t len = active ? e.len - 1u : 0u;
-            in_smem = active && len < kBatchStage;
-            if (in_smem) {   // 8 independent byte loads per lane in flight, then their stores
-                const uint8_t *src = J.arc + e.off + 1;
-                for (uint32_t i0 = 0; i0 < len; i0 += 8u * 32u) {
-                    uint32_t b[8];
-#pragma unroll
-                    for (uint32_t k = 0; k < 8; ++k) {
-                        const uint32_t i = i0 + k * 32u + lane;
-                        b[k] = i < len ? (uint32_t)__ldg(src + i) : 0u;
-                    }
-#pragma unroll
-                    for (uint32_t k = 0; k < 8; ++k) {
-                        const uint32_t i = i0 + k * 32u + lane;
-                        if (i < len) stage[i] = (uint8_t)b[k];
-                    }
-                }
-                if (lane == 0) stage[len] = 0;
-            }
+            in_smem = active && len + kStagePad <= kBatchStage;
+            if (in_smem) stage_stream(stage, J.arc + e.off + 1, len, lane);
             __syncwarp();
             if (lane != 0) continue;
         }

@@ -90,25 +90,20 @@ __global__ void __launch_bounds__(1024) k_scan_u64(uint64_t *v, uint64_t n, uint
     if (tid == 0 && total) *total = carry_s;
 }
 
-// Stream bytes the latency path stages in shared memory (with the zero byte
-// after them, within the 48 KiB a launch may take without opting in; four
-// such CTAs per SM at most).
-constexpr uint32_t kLatStage = 40u * 1024u;
-
-// One warp per CTA, G atoms per warp (rc_lanes_for): G = 1 runs a scalar
-// decoder on lane 0 (the latency decoder when `lat`), G > 1 the lockstep
-// decoder on lanes 0..G-1. With J.order (G = 1 only), CTA i decodes the i-th
-// atom of the payload-length order. With `lat` the whole warp first copies the
-// atom's stream into shared memory (kLatStage bytes of dynamic shared memory:
-// streams that do not fit are read from global memory by
-// rc_decode_levels_lat).
-__global__ void __launch_bounds__(32) k_rc_decode(DecodeJob J, uint32_t G, uint32_t lat) {
-    extern __shared__ uint8_t stage[];
+// One warp per CTA, G atoms per warp (rc_lanes_for): G = 1 runs a one-atom
+// decoder on lane 0, G > 1 the lockstep decoder on lanes 0..G-1. With J.order
+// (G = 1 only), CTA i decodes the i-th atom of the payload-length order. With
+// `stage` bytes of dynamic shared memory (G = 1) the whole warp first copies the
+// atom's stream there, for rc_decode_levels_sm; streams that do not fit are read
+// from global memory (rc_decode_levels_lat; without staging the compact
+// rc_decode_levels_lane).
+__global__ void __launch_bounds__(32) k_rc_decode(DecodeJob J, uint32_t G, uint32_t stage_bytes) {
+    extern __shared__ __align__(16) uint8_t stage[];
     __shared__ uint32_t bstart[9];
     if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
     __syncthreads();
     const uint32_t lane = threadIdx.x;
-    const bool staged = G == 1 && lat;
+    const bool staged = G == 1 && stage_bytes;
     if (G == 1 && !staged && lane != 0) return;
     const uint32_t slot = G == 1 ? 0u : lane;   // (G = 1: every lane of a staging warp takes lane 0's atom)
     uint64_t t = (uint64_t)blockIdx.x * G + slot;
@@ -128,23 +123,9 @@ __global__ void __launch_bounds__(32) k_rc_decode(DecodeJob J, uint32_t G, uint3
     bool in_smem = false;
     if (staged) {
         const uint32_t len = active ? e.len - 1u : 0u;
-        in_smem = active && len < kLatStage;
-        if (in_smem) {   // 8 independent byte loads per lane in flight, then their stores
-            const uint8_t *src = J.arc + e.off + 1;
-            for (uint32_t i0 = 0; i0 < len; i0 += 8u * 32u) {
-                uint32_t b[8];
-#pragma unroll
-                for (uint32_t k = 0; k < 8; ++k) {
-                    const uint32_t i = i0 + k * 32u + lane;
-                    b[k] = i < len ? (uint32_t)__ldg(src + i) : 0u;
-                }
-#pragma unroll
-                for (uint32_t k = 0; k < 8; ++k) {
-                    const uint32_t i = i0 + k * 32u + lane;
-                    if (i < len) stage[i] = (uint8_t)b[k];
-                }
-            }
-            if (lane == 0) stage[len] = 0;
+        in_smem = active && len + kStagePad <= stage_bytes;
+        if (in_smem) {
+            stage_stream(stage, J.arc + e.off + 1, len, lane);
             __syncwarp();
         }
         if (lane != 0) return;
@@ -164,7 +145,7 @@ __global__ void __launch_bounds__(32) k_rc_decode(DecodeJob J, uint32_t G, uint3
     int bad = 0;
     if (G == 1) {
         if (in_smem) bad = rc_decode_levels_sm(stage, e.len - 1, bstart, sink);
-        else if (active && lat) bad = rc_decode_levels_lat(J.arc + e.off + 1, e.len - 1, bstart, sink);
+        else if (active && stage_bytes) bad = rc_decode_levels_lat(J.arc + e.off + 1, e.len - 1, bstart, sink);
         else if (active) bad = rc_decode_levels_lane(J.arc + e.off + 1, e.len - 1, bstart, sink);
     } else {
         bad = rc_decode_levels_warp(J.arc + e.off + 1, active ? e.len - 1 : 0u, active, bstart, sink);
@@ -324,10 +305,28 @@ static void launch_len_sort(const DecodeJob &J, cudaStream_t s) {
     k_len_scatter<<<nb, 256, 0, s>>>(J);
 }
 
+// Shared memory per CTA that stages a stream of a decode of n one-atom warps,
+// the longest payload max_len bytes: enough for every stream if the CTAs that
+// one SM gets then fit it (228 KiB, 1 KiB of it reserved per CTA); with at most
+// one atom per sub-partition as much as fits (a longer stream is read from
+// global memory), above that all or none (0). Measured, range decode of 2,048
+// and 3,072 atoms: staged 3.35 / 3.91 ms at target 10, 1.84 / 2.17 at 20, 0.33 /
+// 0.39 at 100; the compact decoder from global memory 4.40 ms for 2,048 at 10;
+// the per-lane decoder 4.58 / 4.58 at 10.
+constexpr uint32_t kStageMax = 226u * 1024u;
+static uint32_t stage_bytes_for(uint64_t n, uint32_t max_len, uint32_t sms) {
+    const uint64_t per_sm = (n + sms - 1) / sms;
+    const uint64_t room = 228ull * 1024u / per_sm;
+    const uint32_t fit = room > 1280u ? (uint32_t)(room - 1152u < kStageMax ? room - 1152u : kStageMax) & ~127u : 0u;
+    const uint32_t need = (max_len + kStagePad + 127u) & ~127u;
+    if (need <= fit) return need;
+    return n <= 4ull * sms ? fit : 0u;
+}
+
 // The range decode of every PRESENT box atom:
-//   up to one atom per SM sub-partition: latency decoder, one atom per warp;
-//   up to rc_scalar_warps() per sub-partition: scalar decoder, one atom per
-//     warp, longest payload first (the tail is the shortest atoms);
+//   up to rc_scalar_warps() atoms per SM sub-partition: one atom per warp,
+//     longest payload first above one per sub-partition (the tail is the
+//     shortest atoms), the stream staged in shared memory if all streams fit;
 //   above: the per-lane decoder over atoms sorted by payload length, the
 //     rc_solo_for() longest on the latency decoder (k_rc_solo, a warp each,
 //     on the second stream of ev, between its fork and join events).
@@ -360,8 +359,9 @@ static void launch_rc(const DecodeJob &J, int num_sms, cudaStream_t s, const Sta
         Jr.order = nullptr;
         Jr.sort_ctl = nullptr;
     }
-    const uint32_t lat = G == 1 && J.n_atoms <= 4ull * (uint64_t)num_sms ? 1u : 0u;
-    k_rc_decode<<<(unsigned)((J.n_atoms + G - 1) / G), 32, lat ? kLatStage + 16 : 0, s>>>(Jr, G, lat);
+    const uint32_t stage = G == 1 ? stage_bytes_for(J.n_atoms, J.max_len, (uint32_t)num_sms) : 0u;
+    if (stage) smem_attr((const void *)k_rc_decode, (int)kStageMax);
+    k_rc_decode<<<(unsigned)((J.n_atoms + G - 1) / G), 32, stage, s>>>(Jr, G, stage);
 }
 
 // Box atom t: dequantise + inverse transform + crop into the box raster, by NT

@@ -31,6 +31,7 @@ struct DecodeJob {
     unsigned long long *nnz_total;   // coefficient-list entries written (sum over atoms)
     uint32_t band_start[9];      // first scan position of each significance band
     uint64_t t_lo, t_hi;         // box atoms the inverse transform launch covers
+    uint32_t max_len;            // longest payload of the box's PRESENT atoms (sizes the staged streams)
     uint32_t box_table;          // 1: atoms[] is indexed by box atom (staged decode), 0: by LOD raster
     // per-lane range decoder of large decodes (optional; NULL: the warp decoders):
     uint32_t *order;             // n_atoms slots: PRESENT box atoms, longest payload first
@@ -96,9 +97,9 @@ struct BatchShape {              // tunables the autotuner chooses among
 // scalar decoder, whose latency per atom is the lowest. One atom per warp while
 // that makes at most `scalar_warps` warps per SM sub-partition (4 per SM);
 // above that the plain decode path runs the per-lane decoder (k_rc_lanes: all
-// 32 lanes of a warp, each its own atom; measured on GB300 it overtakes the
-// scalar decoder between 2,048 and 4,096 atoms, and at 9,728 t10 atoms it
-// takes 5.4 ms against 11.8 ms). The batched path still runs the lockstep
+// 32 lanes of a warp, each its own atom; at target 10 it takes 4.6 ms from a
+// thousand to ten thousand atoms, where the one-atom decoder goes from 2.5 ms at
+// 608 over 3.9 at 3,072 to 4.9 at 4,864). The batched path still runs the lockstep
 // decoder for G > 1: the fewest warps per sub-partition k that keep a warp at
 // 32 atoms or fewer, the atoms spread evenly over k warps per sub-partition.
 __host__ __device__ inline uint32_t rc_lanes_for(uint64_t n_atoms, uint32_t sms, uint32_t scalar_warps) {
@@ -108,7 +109,7 @@ __host__ __device__ inline uint32_t rc_lanes_for(uint64_t n_atoms, uint32_t sms,
     const uint64_t g = (n_atoms + k * slots - 1) / (k * slots);
     return g < 2 ? 2u : (uint32_t)g;
 }
-constexpr uint32_t kRcScalarWarpsDefault = 8;   // measured crossover with the per-lane decoder: 3-5k atoms
+constexpr uint32_t kRcScalarWarpsDefault = 8;   // as many one-warp CTAs as an SM holds; about where the per-lane decoder takes over
 // the plain decode path puts atoms in payload-length order (and needs the order
 // buffer) above one atom per SM sub-partition
 __host__ __device__ inline bool rc_sorts(uint64_t n_atoms, uint32_t sms) { return n_atoms > 4ull * sms; }

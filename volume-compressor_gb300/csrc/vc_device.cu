@@ -761,6 +761,7 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
     J.arc = arc;
     J.atoms = atoms;
     J.box_table = box_table;
+    J.max_len = r->max_len;
     J.acx = r->acx; J.acy = r->acy;
     J.bax = r->bax; J.bay = r->bay; J.baz = r->baz; J.bnx = r->bnx; J.bny = r->bny;
     J.n_atoms = n;

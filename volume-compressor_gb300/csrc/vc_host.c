@@ -659,15 +659,19 @@ static vc_status decode_box_streamed(vc_archive *a, int lod, vc_box b, uint8_t *
     if (e) { st = (vc_status)e; report("streamed decode: %s", vcd_last_error()); goto out; }
     if (f.fail < nb) nb = f.fail;
     uint64_t cap = 0, bytes = 0, present = 0;
+    uint32_t longest = 0;
     for (uint64_t p = 0; p < np && pidx[p] < nb; ++p) {
+        const uint32_t len = tab[pidx[p]].len;
         cap += entry_cap(&tab[pidx[p]]);
-        bytes += tab[pidx[p]].len;
+        bytes += len;
+        if (len > longest) longest = len;
         ++present;
     }
     r.n_atoms = nb;
     r.cap_total = cap;
     r.payload_bytes = bytes;
     r.present = present;
+    r.max_len = longest;
     if (n_present) *n_present = present;
     e = vcd_decode_staged(a->sdev, &r, 0, arena_off, pay, out_dev, out, out_bytes);
     if (e && e != VC_ERR_FORMAT) report("streamed decode: %s", vcd_last_error());
@@ -696,18 +700,25 @@ static vc_status decode_box(vc_archive *a, int lod, vc_box b, uint8_t *out, uint
     r.bax = b.x0 / 32; r.bay = b.y0 / 32; r.baz = b.z0 / 32;
     r.bnx = (b.x1 - 1) / 32 - r.bax + 1; r.bny = (b.y1 - 1) / 32 - r.bay + 1; r.bnz = (b.z1 - 1) / 32 - r.baz + 1;
     uint64_t n = (uint64_t)r.bnx * r.bny * r.bnz, cap = 0, i = 0, pay = 0, present = 0;
+    uint32_t longest = 0;
     vc_status st = VC_OK;
     for (uint32_t z = 0; z < r.bnz && st == VC_OK; ++z)
         for (uint32_t y = 0; y < r.bny && st == VC_OK; ++y)
             for (uint32_t x = 0; x < r.bnx; ++x, ++i) {
                 const vcd_atom *t = &r.atoms[((uint64_t)(r.baz + z) * r.acy + (r.bay + y)) * r.acx + r.bax + x];
                 if (t->kind == VCD_BAD) { st = VC_ERR_FORMAT; break; }
-                if (t->kind == VCD_PRESENT) { cap += entry_cap(t); pay += t->len; ++present; }
+                if (t->kind == VCD_PRESENT) {
+                    cap += entry_cap(t);
+                    pay += t->len;
+                    if (t->len > longest) longest = t->len;
+                    ++present;
+                }
             }
     r.n_atoms = st == VC_OK ? n : i;
     r.cap_total = cap;
     r.payload_bytes = pay;
     r.present = present;
+    r.max_len = longest;
     size_t bytes = (size_t)(b.x1 - b.x0) * (b.y1 - b.y0) * (b.z1 - b.z0);
     int rc = vcd_decode_region(a->dev, &r, out_dev, out, bytes);
     if (rc == VC_ERR_FORMAT || st == VC_ERR_FORMAT) return VC_ERR_FORMAT;

@@ -61,6 +61,7 @@ typedef struct {
     uint64_t cap_total;         // sum of entry capacities of those atoms
     uint64_t payload_bytes;     // sum of their payload lengths (for profiling)
     uint64_t present;           // PRESENT atoms among them
+    uint32_t max_len;           // their longest payload
     int lod;
 } vcd_region;
 

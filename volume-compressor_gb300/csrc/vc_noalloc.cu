@@ -97,12 +97,14 @@ VC_API int vcg_decode_atoms_noalloc(const uint8_t *payload_dev, size_t payload_b
     if (n_atoms == 0) return 0;
     vcd_atom atoms[NA_MAX_ATOMS];
     memset(atoms, 0, sizeof atoms);
+    uint32_t longest = 0;
     for (uint32_t i = 0; i < n_atoms; ++i) {
         if (lengths[i] == 0) { atoms[i].kind = VCD_EMPTY; continue; }
         if (offsets[i] > payload_bytes || lengths[i] > payload_bytes - offsets[i]) return 1;   // VC_ERR_FORMAT
         atoms[i].kind = VCD_PRESENT;
         atoms[i].off = offsets[i];
         atoms[i].len = lengths[i];
+        if (lengths[i] > longest) longest = lengths[i];
     }
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -132,6 +134,7 @@ VC_API int vcg_decode_atoms_noalloc(const uint8_t *payload_dev, size_t payload_b
     J.acx = 1; J.acy = 1;                       // atoms stacked along z: atom i = voxels z in [32i, 32i+32)
     J.bnx = 1; J.bny = 1;
     J.n_atoms = n_atoms;
+    J.max_len = longest;
     J.x1 = 32; J.y1 = 32; J.z1 = 32 * n_atoms;
     J.out = out_dev;
     J.ox = 32; J.oy = 32;
