@@ -1,5 +1,5 @@
-// Decode kernels: per-atom list capacities + scan, range-decode lanes, and the
-// fused dequantise + inverse DCT-32 + crop.
+// Decode kernels: per-atom list capacities + scan, range decoders, and the
+// dequantise + inverse DCT-32 + crop.
 //
 //   k_caps       one thread per box atom: coefficient-list capacity
 //   k_scan_u64   one CTA: exclusive scan of the capacities (list placement)
@@ -7,25 +7,24 @@
 //                payload into (scan position, level) pairs (src/vc/vc.c:545-560);
 //                one atom per warp for small decodes, a warp of atoms in
 //                lockstep for large ones
-//   k_idct       one CTA per atom (persistent over the box): scatter levels into
-//                a 32x32x32 i32 tile in shared memory, dequantise while loading
-//                each z-slab (src/vc/vc.c:327-338), inverse passes along x and y
-//                per slab (warp per slab, lane per line), then along z (lane per
-//                column), add dc, clamp to u8 and store the cropped voxels
-//                (src/vc/vc.c:219-229, 1535-1555)
+//   k_idct       persistent, one CTA per SM: levels dequantised
+//                (src/vc/vc.c:327-338), inverse passes along x, y, z on the tensor
+//                cores (idct_mma.cuh), dc added, clamped, cropped into the box
+//                (src/vc/vc.c:219-229, 1535-1555); atoms that cannot go there,
+//                and small decodes (k_idct_bf), take the butterfly on a 32x32x32
+//                i32 tile in shared memory (idct_tile.cuh)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "dct32.cuh"
 #include "kernels.cuh"
+#include "idct_mma.cuh"
 #include "idct_tile.cuh"
 #include "rangecoder.cuh"
 #include "rc_lanes.cuh"
 
 namespace vcg {
 
-constexpr int kIdctThreads = 512;   // 16 warps per atom (measured faster than 8 on GB300)
-constexpr size_t kIdctSmem = kIdctTileBytes;
 
 __global__ void k_caps(DecodeJob J) {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -364,8 +363,9 @@ static void launch_rc(const DecodeJob &J, int num_sms, cudaStream_t s, const Sta
     k_rc_decode<<<(unsigned)((J.n_atoms + G - 1) / G), 32, stage, s>>>(Jr, G, stage);
 }
 
-// Box atom t: dequantise + inverse transform + crop into the box raster, by NT
-// threads (tid = 0..NT-1) that meet at barrier BAR (tile_sync); ends with one.
+// Box atom t without the tensor cores: zeros (ABSENT, KNOWN_ZERO, malformed), or
+// dequantise + butterfly + crop into the box raster, by NT threads (tid =
+// 0..NT-1) that meet at barrier BAR (tile_sync); ends with one.
 template <int NT, int BAR>
 __device__ __forceinline__ void idct_atom(const DecodeJob &J, uint64_t t, int32_t *T, const int32_t *dqs,
                                           const int32_t *dqb, const uint32_t *alt, int tid) {
@@ -377,15 +377,13 @@ __device__ __forceinline__ void idct_atom(const DecodeJob &J, uint64_t t, int32_
     const uint32_t gx = ax * 32, gy = ay * 32, gz = az * 32;
     k.set(gx, gy, gz, J.x0, J.y0, J.z0, J.x1, J.y1, J.z1);
     uint8_t *obase = J.out + ((uint64_t)(gz + k.lz0 - J.z0) * J.oy + (gy + k.ly0 - J.y0)) * J.ox + (gx + k.lx0 - J.x0);
-    // (BAR != 0: inside the fused decode, whose lists and counts this kernel wrote)
-    const uint32_t c = e.kind == VCD_PRESENT ? (BAR ? __ldcg(J.cnt + t) : J.cnt[t]) : kEntBad;
+    const uint32_t c = e.kind == VCD_PRESENT ? J.cnt[t] : kEntBad;
     if (e.kind != VCD_PRESENT || (c & kEntBad)) {   // ABSENT / KNOWN_ZERO -> zeros
         zero_window<NT>(obase, J.ox, J.oy, k, (uint32_t)tid);
         return;
     }
     const int32_t dc = J.arc[e.off];
-    idct_tile_xy<NT, BAR, BAR != 0, BAR != 0>(T, J.arc, e, c, J.ent + J.ent_off[t], J.scan, J.band_start, dqs, dqb,
-                                               alt, tid);
+    idct_tile_xy<NT, BAR>(T, J.arc, e, c, J.ent + J.ent_off[t], J.scan, J.band_start, dqs, dqb, alt, tid);
     const bool full = k.lz0 == 0 && k.lz1 == 32;
     for (int y = warp; y < 32; y += NT / 32) {
         int32_t o[32];
@@ -395,173 +393,75 @@ __device__ __forceinline__ void idct_atom(const DecodeJob &J, uint64_t t, int32_
     }
     tile_sync<NT, BAR>();
 }
+__device__ __noinline__ void idct_atom_other(const DecodeJob &J, uint64_t t, int32_t *T, int tid) {   // in k_idct
+    idct_atom<kMmaThreads, kMmaBar>(J, t, T, J.dq->step, J.dq->bias, J.alt_mask, tid);
+}
 
-__global__ void __launch_bounds__(kIdctThreads, 1) k_idct(DecodeJob J) {
+// Few atoms: the butterfly on the CUDA cores. With one to three atoms per SM the
+// tensor-core kernel's start (TMEM, matrix pieces, first lists) and the chain of
+// its passes are not hidden: one atom 33 us against 20, 576 atoms 68 against 66,
+// 4,096 atoms 0.36 ms against 0.58.
+constexpr int kBfThreads = 512;   // 16 warps per atom (measured faster than 8 on GB300)
+constexpr uint64_t kMmaAtomsPerSm = 4;
+__global__ void __launch_bounds__(kBfThreads, 1) k_idct_bf(DecodeJob J) {
     extern __shared__ int32_t T[];   // 32 slabs x padded 32x32 (idct_tile.cuh)
     __shared__ int32_t dqs[VCD_NCLASS], dqb[VCD_NCLASS];
     __shared__ uint32_t alt[1024];
     const int tid = threadIdx.x;
-    for (int i = tid; i < VCD_NCLASS; i += kIdctThreads) { dqs[i] = J.dq->step[i]; dqb[i] = J.dq->bias[i]; }
-    for (int i = tid; i < 1024; i += kIdctThreads) alt[i] = J.alt_mask[i];
+    for (int i = tid; i < VCD_NCLASS; i += kBfThreads) { dqs[i] = J.dq->step[i]; dqb[i] = J.dq->bias[i]; }
+    for (int i = tid; i < 1024; i += kBfThreads) alt[i] = J.alt_mask[i];
     __syncthreads();
-    for (uint64_t t = J.t_lo + blockIdx.x; t < J.t_hi; t += gridDim.x) idct_atom<kIdctThreads, 0>(J, t, T, dqs, dqb, alt, tid);
+    for (uint64_t t = J.t_lo + blockIdx.x; t < J.t_hi; t += gridDim.x) idct_atom<kBfThreads, 0>(J, t, T, dqs, dqb, alt, tid);
 }
 
-// ---- fused decode: range decode and inverse transform in one persistent
-// kernel, one CTA per SM. Each CTA owns the entries c, c + G, c + 2G, ... of
-// the payload-length order (G CTAs), so every CTA gets the same mix of long
-// and short atoms. Its first 8 warps decode them: the CTA's head (entry c, its
-// longest atom) on one lane of the 8th warp with the latency decoder (a
-// decision in about 50 ns against about 110 ns for a step of the per-lane
-// decoder in a full warp, so the longest atoms no longer set the coder's end),
-// the others with the per-lane decoder on 7 warps (lane j takes the CTA's
-// entries 1 + j, 1 + j + 224, ...); whenever an atom is decoded it is published
-// in the CTA's queue. The other 8 warps transform the
-// queued atoms in that order (ABSENT / KNOWN_ZERO atoms are queued at the
-// start), so the transforms of finished atoms run while the coder is still busy
-// with the longer ones: the integer-multiply pipe of the transform and the ALU
-// work of the coder share the SM instead of running one after the other. Only
-// warps of the same CTA wait for one another; a wait that exceeds kFusedSpin
-// polls sets *fail and the transform warps stop.
-constexpr int kFusedRcThreads = 256;   // 8 decoding warps
-constexpr int kFusedLaneThreads = kFusedRcThreads - 32;   // 7 of them per-lane; the 8th: the CTA's head atom
-constexpr int kFusedTxThreads = 256;   // 8 transforming warps
-constexpr int kFusedThreads = kFusedRcThreads + kFusedTxThreads;
-constexpr uint32_t kQueueEmpty = 0xFFFFFFFFu;
-constexpr uint64_t kFusedSpin = 1ull << 24;   // x 256 ns sleeps: about 4 s
+// Dynamic shared memory of k_idct from a 1024-byte boundary on: the operand of
+// the tensor-core passes, or the butterfly's tile in its place; the matrix
+// pieces; the feeders' ring.
+constexpr uint32_t kIdctB = (uint32_t)((kIdctTileBytes + 1023) & ~(size_t)1023);
+constexpr size_t kIdctSmem = 1024 + kIdctB + kMmaB + kMmaRing;
+static_assert(kMmaA <= kIdctB, "the matrix pieces lie behind the operand and the tile");
 
-__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// queue: G x per slots, CTA c's at [c * per, c * per + per), preset to kQueueEmpty
-__global__ void __launch_bounds__(kFusedThreads, 1) k_decode_fused(DecodeJob J, uint32_t *queue, uint32_t per,
-                                                                    uint32_t *fail) {
-    extern __shared__ int32_t T[];   // transform tile
-    __shared__ uint32_t bstart[10];   // the band table and a copy of its end (RcLane)
-    __shared__ uint32_t S[kFusedRcThreads / 32][kLaneRows * 32];
-    __shared__ int32_t dqs[VCD_NCLASS], dqb[VCD_NCLASS];
-    __shared__ uint32_t alt[1024];
-    __shared__ uint32_t q_tail;   // slots of this CTA's queue handed out
-    __shared__ uint32_t cur[2];   // atom of the transform's current iteration (double-buffered)
+// Persistent: one CTA per SM, atoms blockIdx.x, blockIdx.x + grid, ...
+__global__ void __launch_bounds__(kMmaCta, 1) k_idct(DecodeJob J) {
+    extern __shared__ uint8_t dyn[];
+    __shared__ __align__(16) MmaShared M;
+    uint8_t *A = dyn + ((1024u - (smem_u32(dyn) & 1023u)) & 1023u), *B = A + kIdctB, *ring = B + kMmaB;
     const int tid = threadIdx.x;
-    if (tid < 10) bstart[tid] = J.band_start[tid < 9 ? tid : 8];
-    for (int i = tid; i < VCD_NCLASS; i += kFusedThreads) { dqs[i] = J.dq->step[i]; dqb[i] = J.dq->bias[i]; }
-    for (int i = tid; i < 1024; i += kFusedThreads) alt[i] = J.alt_mask[i];
-    if (tid == 0) q_tail = 0;
-    __syncthreads();
-    const uint32_t G = gridDim.x, cta = blockIdx.x;
-    const uint32_t n = (uint32_t)J.n_atoms, n_present = J.sort_ctl[kSortBuckets];
-    const uint32_t n_cta = cta < n ? (n - 1 - cta) / G + 1 : 0;
-    const uint32_t np_cta = cta < n_present ? (n_present - 1 - cta) / G + 1 : 0;
-    uint32_t *Q = queue + (uint64_t)cta * per;
-    if (tid < kFusedRcThreads) {
-        for (uint32_t k = np_cta + tid; k < n_cta; k += kFusedRcThreads)   // nothing to decode
-            atomicExch(Q + atomicAdd(&q_tail, 1u), J.order[cta + k * G]);
-        if (tid >= kFusedLaneThreads) {   // the head: the CTA's longest atom, alone on one lane
-            if (tid == kFusedLaneThreads && np_cta) {
-                const uint32_t t = J.order[cta];
-                uint32_t az, ay, ax;
-                box_atom(J, t, az, ay, ax);
-                const vcd_atom e = J.atoms[job_atom(J, t, az, ay, ax)];
-                uint32_t cap = 8u * (e.len - 1u) + 64u;
-                if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
-                uint32_t *dst = J.ent + J.ent_off[t];
-                uint32_t cnt = 0;
-                auto sink = [&](uint32_t p, uint32_t lv) {
-                    if (cnt < cap) dst[cnt] = p | (lv << 16);
-                    ++cnt;
-                };
-                const int bad = rc_decode_levels_lat(J.arc + e.off + 1, e.len - 1u, bstart, sink);
-                const uint32_t m = cnt > cap ? cap : cnt;
-                J.cnt[t] = m | (cnt > cap ? kEntOverflow : 0u) | (bad ? kEntBad : 0u);
-                atomicAdd(J.nnz_total, (unsigned long long)m);
-                if (bad) atomicMin(J.err, t);
-                __threadfence();
-                atomicExch(Q + atomicAdd(&q_tail, 1u), t);
-            }
-            return;
-        }
-        uint32_t *Sl = &S[tid >> 5][tid & 31];
-        uint32_t k = 1u + (uint32_t)tid, t = 0, cap = 0;   // the CTA's entries after its head
-        bool have = false;
-        RcLane L;
-        auto start = [&]() {   // the lane's next atom, if any
-            have = k < np_cta;
-            vcd_atom e = {};
-            uint32_t *dst = J.ent;
-            if (have) {
-                t = J.order[cta + k * G];
-                uint32_t az, ay, ax;
-                box_atom(J, t, az, ay, ax);
-                e = J.atoms[job_atom(J, t, az, ay, ax)];
-                cap = 8u * (e.len - 1u) + 64u;
-                if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
-                dst = J.ent + J.ent_off[t];
-            }
-            L.init(J.arc + e.off + 1, e.len - 1u, have, bstart, Sl, 32, dst, cap);
-        };
-        start();
-        while (__any_sync(0xFFFFFFFFu, have)) {
-            L.step(bstart, Sl, 32);
-            if (have && L.c == kLaneDone) {   // finished: counts, then publish the atom
-                const uint32_t m = L.n > cap ? cap : L.n;
-                J.cnt[t] = m | (L.n > cap ? kEntOverflow : 0u) | (L.bad ? kEntBad : 0u);
-                atomicAdd(J.nnz_total, (unsigned long long)m);
-                if (L.bad) atomicMin(J.err, t);
-                __threadfence();
-                atomicExch(Q + atomicAdd(&q_tail, 1u), t);
-                k += kFusedLaneThreads;
-                start();
-            }
-        }
+    mma_setup(M, B);
+    if (tid >= kMmaFeed) {
+        mma_feed(M, ring, J.dq, J.place, [&](uint32_t i, MmaAtom &a) {
+            const uint64_t t = J.t_lo + blockIdx.x + (uint64_t)i * gridDim.x;
+            if (t >= J.t_hi) return false;
+            uint32_t az, ay, ax;
+            box_atom(J, t, az, ay, ax);
+            const vcd_atom e = J.atoms[job_atom(J, t, az, ay, ax)];
+            a.id = t;
+            a.lod = 0;
+            a.src = J.ent + J.ent_off[t];
+            const uint32_t c = e.kind == VCD_PRESENT ? J.cnt[t] : kEntBad;
+            a.n = c & kEntMask;
+            a.tensor = !(c & (kEntBad | kEntOverflow));
+            a.dc = a.tensor ? (int32_t)J.arc[e.off] : 0;
+            const uint32_t gx = ax * 32, gy = ay * 32, gz = az * 32;
+            a.crop.set(gx, gy, gz, J.x0, J.y0, J.z0, J.x1, J.y1, J.z1);
+            a.out = J.out + ((uint64_t)(gz + a.crop.lz0 - J.z0) * J.oy + (gy + a.crop.ly0 - J.y0)) * J.ox +
+                    (gx + a.crop.lx0 - J.x0);
+            return true;
+        });
+    } else if (tid >= kMmaIssuer) {
+        if (tid == kMmaIssuer) mma_issue(M, umma_lo(smem_u32(A)), umma_lo(smem_u32(B)));
     } else {
-        const int tt = tid - kFusedRcThreads;
-        for (uint32_t k = 0; k < n_cta; ++k) {
-            if (tt == 0) {
-                uint32_t v = ld_acquire_u32(Q + k);
-                for (uint64_t spins = 0; v == kQueueEmpty; v = ld_acquire_u32(Q + k)) {
-                    if (++spins > kFusedSpin) {
-                        atomicExch(fail, 1u);
-                        break;
-                    }
-                    __nanosleep(256);
-                }
-                cur[k & 1] = v;
-            }
-            tile_sync<kFusedTxThreads, 1>();
-            const uint32_t t = cur[k & 1];
-            if (t == kQueueEmpty) break;   // gave up waiting (every transform thread sees it)
-            __threadfence();
-            idct_atom<kFusedTxThreads, 1>(J, t, T, dqs, dqb, alt, tt);
-        }
+        const bool ok = mma_atoms(
+            A, M, ring,
+            [&](const MmaAtom &a, int y, int x, int z, uint32_t (&o)[16]) {
+                store_magic(a.out, J.ox, J.oy, a.crop, y, x, z, o, a.dc);
+            },
+            [&](const MmaAtom &a, uint8_t *T) {   // zeros, a list that overflowed, coefficients too large
+                idct_atom_other(J, a.id, reinterpret_cast<int32_t *>(T), tid);
+            });
+        if (!ok) atomicExch(J.fail, 1u);   // a wait ran out: the call fails
     }
-}
-
-// Fused range decode + transform of a whole box: above one atom per warp (the
-// per-lane decoder's range) with an order buffer; queue: per-CTA slots
-// (decode_fused_queue_words(n) words), fail: a zeroed word. Returns false when
-// the box takes the separate kernels instead.
-bool launch_decode_fused(const DecodeJob &J, int num_sms, cudaStream_t s, uint32_t *queue, uint32_t *fail,
-                         const StageEvents *ev) {
-    if (!J.order || !J.sort_ctl || !queue || rc_lanes_for(J.n_atoms, (uint32_t)num_sms, rc_scalar_warps()) <= 1)
-        return false;
-    const uint32_t G = (uint32_t)num_sms;
-    const uint32_t per = (uint32_t)((J.n_atoms + G - 1) / G);
-    if (ev) cudaEventRecord(ev->ev[0], s);
-    const unsigned nb = (unsigned)((J.n_atoms + 127) / 128);
-    k_caps<<<nb, 128, 0, s>>>(J);
-    launch_scan_u64(J.ent_off, J.n_atoms, 0, nullptr, s);
-    if (ev) cudaEventRecord(ev->ev[1], s);
-    launch_len_sort(J, s);
-    cudaMemsetAsync(queue, 0xFF, (size_t)G * per * 4, s);
-    if (ev) cudaEventRecord(ev->ev[2], s);
-    smem_attr((const void *)k_decode_fused, (int)kIdctSmem);
-    k_decode_fused<<<G, kFusedThreads, kIdctSmem, s>>>(J, queue, per, fail);
-    if (ev) cudaEventRecord(ev->ev[3], s);
-    return true;
+    mma_release(M);
 }
 
 void launch_scan_u64(uint64_t *v, uint64_t n, uint64_t base, uint64_t *total, cudaStream_t s) {
@@ -570,13 +470,18 @@ void launch_scan_u64(uint64_t *v, uint64_t n, uint64_t base, uint64_t *total, cu
 
 void launch_idct(const DecodeJob &J, int num_sms, cudaStream_t s, uint64_t t_lo, uint64_t t_hi) {
     if (t_hi <= t_lo) return;
-    smem_attr((const void *)k_idct, (int)kIdctSmem);
     DecodeJob Jr = J;
     Jr.t_lo = t_lo;
     Jr.t_hi = t_hi;
     const uint64_t n = t_hi - t_lo;
     const uint64_t grid = n < (uint64_t)num_sms ? n : (uint64_t)num_sms;
-    k_idct<<<(unsigned)grid, kIdctThreads, kIdctSmem, s>>>(Jr);
+    if (n < kMmaAtomsPerSm * (uint64_t)num_sms) {
+        smem_attr((const void *)k_idct_bf, (int)kIdctTileBytes);
+        k_idct_bf<<<(unsigned)grid, kBfThreads, kIdctTileBytes, s>>>(Jr);
+    } else {
+        smem_attr((const void *)k_idct, (int)kIdctSmem);
+        k_idct<<<(unsigned)grid, kMmaCta, kIdctSmem, s>>>(Jr);
+    }
 }
 
 void launch_decode_lists(const DecodeJob &J, int num_sms, cudaStream_t s) {

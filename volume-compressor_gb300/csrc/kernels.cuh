@@ -27,7 +27,9 @@ struct DecodeJob {
     const vcd_dq *dq;            // dequant tables of the LOD
     const uint32_t *alt_mask;    // step-class alternate bits
     const uint16_t *scan;        // scan position -> raster
+    const uint32_t *place;       // scan position -> place and step class (vcd_tables)
     uint32_t *err;               // lowest malformed box atom (atomicMin)
+    uint32_t *fail;              // set when a kernel gave up a wait (zero before)
     unsigned long long *nnz_total;   // coefficient-list entries written (sum over atoms)
     uint32_t band_start[9];      // first scan position of each significance band
     uint64_t t_lo, t_hi;         // box atoms the inverse transform launch covers
@@ -57,9 +59,16 @@ struct StageEvents {
 
 __host__ __device__ inline void box_atom(const DecodeJob &J, uint64_t t, uint32_t &az, uint32_t &ay,
                                          uint32_t &ax) {
-    ax = J.bax + (uint32_t)(t % J.bnx);
-    ay = J.bay + (uint32_t)((t / J.bnx) % J.bny);
-    az = J.baz + (uint32_t)(t / ((uint64_t)J.bnx * J.bny));
+    if (t >> 32) {
+        ax = J.bax + (uint32_t)(t % J.bnx);
+        ay = J.bay + (uint32_t)((t / J.bnx) % J.bny);
+        az = J.baz + (uint32_t)(t / ((uint64_t)J.bnx * J.bny));
+    } else {   // (a 64-bit division is some 70 instructions)
+        const uint32_t row = (uint32_t)t / J.bnx;
+        ax = J.bax + (uint32_t)t % J.bnx;
+        ay = J.bay + row % J.bny;
+        az = J.baz + row / J.bny;
+    }
 }
 
 // ---- batched region decode: every distinct atom of a batch of boxes is decoded
@@ -79,6 +88,7 @@ struct BatchJob {
     const vcd_dq *dq;            // per LOD
     const uint32_t *alt_mask;
     const uint16_t *scan;
+    const uint32_t *place;
     uint32_t *work;              // transform work counter (reset per batch)
     uint32_t *req_err;           // per request: set when one of its atoms is malformed
     uint32_t band_start[9];
@@ -141,13 +151,6 @@ void launch_decode_lists(const DecodeJob &J, int num_sms, cudaStream_t s);
 void launch_scan_u64(uint64_t *v, uint64_t n, uint64_t base, uint64_t *total, cudaStream_t s);
 // exclusive scan of the kSortBuckets length counters in place, their sum after them
 void launch_len_scan(uint32_t *sort_ctl, cudaStream_t s);
-// Range decode and inverse transform of a whole box in one kernel (k_decode_fused)
-// when the box takes the per-lane decoder and J has an order buffer: queue holds
-// n_atoms + num_sms words, fail a word that starts at zero (set if the kernel
-// gave up waiting). Records ev[0..3] like launch_decode. False: not applicable.
-bool launch_decode_fused(const DecodeJob &J, int num_sms, cudaStream_t s, uint32_t *queue, uint32_t *fail,
-                         const StageEvents *ev);
-
 // cudaFuncAttributeMaxDynamicSharedMemorySize of kernel fn, set on the calling
 // thread's current device. The attribute belongs to the device's context, not
 // to the process, so it is set once per (kernel, device) pair.

@@ -720,8 +720,6 @@ cudaError_t vcd_copy_from_host(vcd_ctx *c, void *dst_dev, const void *src, size_
 }
 
 // ---------------------------------------------------------------- decode
-constexpr uint64_t kFusedMaxPayload = 3072;   // mean payload bytes per PRESENT atom of a fused decode
-
 // One box decode from device bytes `arc` and atom table `atoms` (LOD raster, or
 // box order when box_table). last_ms spans from `t0` (or the first stage event).
 static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uint32_t box_table, const vcd_dq *dq,
@@ -745,10 +743,9 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
     }
     p_err = p_ctl;
     void *p_ord = NULL;   // only large decodes use the per-lane range decoder (launch_rc)
-    // [sort counters][order: n][fused-decode queue: n + SMs]
+    // [sort counters][order: n]
     if (rc_sorts(n, (uint32_t)g_dev.num_sms) &&
-        (e = vcd_scratch(c, VCD_BUF_ORD, (2 * n + g_dev.num_sms + sort_ctl_words()) * 4 + 16, &p_ord)) !=
-            cudaSuccess) {
+        (e = vcd_scratch(c, VCD_BUF_ORD, (n + sort_ctl_words()) * 4 + 16, &p_ord)) != cudaSuccess) {
         vcd_set_error("decode scratch", e);
         return vcd_status_of(e);
     }
@@ -774,7 +771,9 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
     J.dq = dq;
     J.alt_mask = g_dev.tables->alt_mask;
     J.scan = g_dev.tables->scan;
+    J.place = g_dev.tables->place;
     J.err = (uint32_t *)p_err;
+    J.fail = (uint32_t *)p_ctl + 1;
     J.nnz_total = (unsigned long long *)((uint8_t *)p_ctl + 8);
     memcpy(J.band_start, g_dev.band_start, sizeof J.band_start);
     if (p_ord) {
@@ -807,7 +806,7 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
     // payload range keeps the exact per-atom copy below)
     // (pageable destinations take the same slabs, copied out through pinned
     // bounce chunks by host threads)
-    bool piped = false, bounce = false, fused = false;
+    bool piped = false, bounce = false;
     const uint64_t layer = (uint64_t)r->bnx * r->bny, layers = layer ? n / layer : 0;
     if (out_host && out_bytes >= (64ull << 20) && n == box_atoms && layers * layer == n && layers >= 2) {
         cudaPointerAttributes pa;
@@ -829,7 +828,10 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
             piped = false;
         } else {
             const uint64_t plane = (uint64_t)J.ox * J.oy;
-            const uint64_t per = (layers + VCD_SLABS - 1) / VCD_SLABS;
+            uint64_t per = (layers + VCD_SLABS - 1) / VCD_SLABS;
+            // (at least four atoms per SM: the transform kernel's start is worth two)
+            const uint64_t least = (4ull * (uint64_t)g_dev.num_sms + layer - 1) / layer;
+            if (per < least) per = least;
             uint64_t slab_end[VCD_SLABS];
             int k = 0;
             for (uint64_t l0 = 0; l0 < layers; l0 += per, ++k) {
@@ -854,23 +856,14 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
             }
         }
     } else {
-        // fused only for light payloads: on GB300 a 1024^3 decode at ~4.4 KB per atom
-        // (target 10) took 12.9 ms fused against 11.6 ms for the two kernels (the
-        // transform warps take issue slots from the latency-bound coder), at ~1 KB
-        // (target 50) 5.9 against ~7 ms and at ~0.5 KB (target 100) 4.0 against 4.5
-        const bool light = r->present && r->payload_bytes <= kFusedMaxPayload * r->present;
-        fused = p_ord && light &&
-                launch_decode_fused(J, g_dev.num_sms, c->stream, J.order + n, (uint32_t *)p_ctl + 1, &ev);
-        if (!fused) {
-            launch_decode_front(J, g_dev.num_sms, c->stream, &ev);
-            if ((e = cudaPeekAtLastError()) != cudaSuccess) {
-                vcd_set_error("decode launch (lists, range decoder)", e);
-                cudaGetLastError();
-                return vcd_status_of(e);
-            }
-            launch_idct(J, g_dev.num_sms, c->stream, 0, n);
-            cudaEventRecord(ev.ev[3], c->stream);
+        launch_decode_front(J, g_dev.num_sms, c->stream, &ev);
+        if ((e = cudaPeekAtLastError()) != cudaSuccess) {
+            vcd_set_error("decode launch (lists, range decoder)", e);
+            cudaGetLastError();
+            return vcd_status_of(e);
         }
+        launch_idct(J, g_dev.num_sms, c->stream, 0, n);
+        cudaEventRecord(ev.ev[3], c->stream);
         if ((e = cudaPeekAtLastError()) != cudaSuccess) {
             vcd_set_error("decode launch (inverse transform)", e);
             cudaGetLastError();
@@ -881,29 +874,24 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
             return vcd_status_of(e);
         }
     }
+    if (piped) cudaMemcpyAsync(ctl_h, p_ctl, 16, cudaMemcpyDeviceToHost, c->stream);   // as the transform left it
     if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess || (piped && (e = cudaStreamSynchronize(c->copy_stream)) != cudaSuccess) ||
         (e = cudaGetLastError()) != cudaSuccess) {
         vcd_set_error("decode kernels", e);
         return vcd_status_of(e);
     }
     c->last_ms = vcd_elapsed(t0 ? t0 : ev.ev[0], ev.ev[3]);
-    if (fused && (ctl_h[0] >> 32) != 0) {   // the fused kernel's transform warps gave up waiting
-        vcd_set_error("fused decode: an atom never reached the transform", cudaSuccess);
+    if ((ctl_h[0] >> 32) != 0) {   // a kernel gave up waiting (for an atom, or for the tensor cores)
+        vcd_set_error("decode: a wait inside a kernel ran out", cudaSuccess);
         return 4;
     }
     if (vcd_prof_on()) {
         const uint64_t nnz = ctl_h[1];
         vcd_prof_add("decode_place", vcd_elapsed(ev.ev[0], ev.ev[1]), n ? 2 : 0, 24 * n, 8 * n, n);
-        if (fused) {   // length sort (three kernels); range decode + transform in one kernel
-            vcd_prof_add("length_sort", vcd_elapsed(ev.ev[1], ev.ev[2]), 3, 16 * n, 8 * n, n);
-            vcd_prof_add("decode_fused", vcd_elapsed(ev.ev[2], ev.ev[3]), 1, r->payload_bytes + 16 * n, out_bytes,
-                         n);
-        } else {
-            // (the per-lane decoder: length sort in three kernels, then the decoder)
-            vcd_prof_add("rc_decode", vcd_elapsed(ev.ev[1], ev.ev[2]), n ? (p_ord ? (solo ? 6 : 4) : 1) : 0,
-                         r->payload_bytes + 16 * n, 4 * nnz, r->present);
-            vcd_prof_add("idct", vcd_elapsed(ev.ev[2], ev.ev[3]), n ? 1 : 0, 4 * nnz + 16 * n, out_bytes, n);
-        }
+        // (the per-lane decoder: length sort in three kernels, then the decoder)
+        vcd_prof_add("rc_decode", vcd_elapsed(ev.ev[1], ev.ev[2]), n ? (p_ord ? (solo ? 6 : 4) : 1) : 0,
+                     r->payload_bytes + 16 * n, 4 * nnz, r->present);
+        vcd_prof_add("idct", vcd_elapsed(ev.ev[2], ev.ev[3]), n ? 1 : 0, 4 * nnz + 16 * n, out_bytes, n);
     }
     const uint32_t err_h = (uint32_t)ctl_h[0];
     const uint64_t good = err_h < n ? err_h : n;   // atoms written before the first bad one

@@ -125,6 +125,14 @@ void vch_tables(vcd_tables *t) {
     uint32_t fill[94];
     memcpy(fill, first, sizeof fill);
     for (uint32_t r = 0; r < 32768; ++r) t->scan[fill[(r >> 10) + ((r >> 5) & 31) + (r & 31)]++] = (uint16_t)r;
+    // operand of rows (kz, ky) of 128 bytes, kx along them in fp16, 16-byte pieces
+    // swizzled by the row
+    for (uint32_t p = 0; p < 32768; ++p) {
+        const uint32_t r = t->scan[p], row = r >> 5, kx = r & 31;
+        const uint32_t at = row * 128 + (((kx >> 3) ^ (row & 7)) << 4) + (kx & 7) * 2;
+        const uint32_t cls = (r >> 10) + ((r >> 5) & 31) + (r & 31) + 94 * ((t->alt_mask[r >> 5] >> (r & 31)) & 1);
+        t->place[p] = at | (cls << 17);
+    }
     // rank_base[f][kz]: scan position of the first index with frequency f and
     // plane kz (the one with the smallest valid ky)
     for (int f = 0; f < 94; ++f) {

@@ -45,6 +45,9 @@ typedef struct {
 typedef struct {
     uint32_t alt_mask[1024];   // bit i: raster index i uses the alternate step value
     uint16_t scan[32768];      // scan position -> raster index
+    // scan position -> place of the coefficient in the tensor-core transform's
+    // first operand (idct_mma.cuh) | step class << 17
+    uint32_t place[32768];
     uint16_t rank_base[94 * 32];  // scan position of (f, kz, ky = max(0, f-kz-31))
     uint32_t band_start[9];    // first scan position of each significance band, [8] = 32768
 } vcd_tables;

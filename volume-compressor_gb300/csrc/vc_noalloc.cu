@@ -32,7 +32,8 @@ constexpr size_t kNaAtoms = kNaCtl + 256;                                  // 64
 constexpr size_t kNaDq = kNaAtoms + NA_MAX_ATOMS * sizeof(vcd_atom);       // vcd_dq
 constexpr size_t kNaScan = kNaDq + ((sizeof(vcd_dq) + 255) / 256) * 256;   // scan order: 32768 x u16
 constexpr size_t kNaAlt = kNaScan + 32768 * 2;                             // step-class bits: 1024 x u32
-constexpr size_t kNaBytes = kNaAlt + 4096;                                 // ~8.07 MiB
+constexpr size_t kNaPlace = kNaAlt + 4096;                                 // places and step classes: 32768 x u32
+constexpr size_t kNaBytes = kNaPlace + 32768 * 4;                          // ~8.2 MiB
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
@@ -52,7 +53,7 @@ static int na_setup(int dev, uint8_t **base, int *sms) {
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess) {
             // constant parts: scan order, step-class bits, fixed list offsets
-            static vcd_tables t;   // host staging (68 KiB), filled once
+            static vcd_tables t;   // host staging, filled once
             vch_tables(&t);
             memcpy(g_na_band, t.band_start, sizeof g_na_band);
             uint64_t offs[NA_MAX_ATOMS];
@@ -60,6 +61,7 @@ static int na_setup(int dev, uint8_t **base, int *sms) {
             uint8_t *b = (uint8_t *)p;
             e = cudaMemcpy(b + kNaScan, t.scan, sizeof t.scan, cudaMemcpyHostToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(b + kNaAlt, t.alt_mask, sizeof t.alt_mask, cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = cudaMemcpy(b + kNaPlace, t.place, sizeof t.place, cudaMemcpyHostToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(b + kNaOff, offs, sizeof offs, cudaMemcpyHostToDevice);
         }
         if (e != cudaSuccess) {
@@ -144,7 +146,9 @@ VC_API int vcg_decode_atoms_noalloc(const uint8_t *payload_dev, size_t payload_b
     J.dq = reinterpret_cast<const vcd_dq *>(base + kNaDq);
     J.alt_mask = reinterpret_cast<const uint32_t *>(base + kNaAlt);
     J.scan = reinterpret_cast<const uint16_t *>(base + kNaScan);
+    J.place = reinterpret_cast<const uint32_t *>(base + kNaPlace);
     J.err = reinterpret_cast<uint32_t *>(base + kNaCtl);
+    J.fail = J.err + 1;
     J.nnz_total = reinterpret_cast<unsigned long long *>(base + kNaCtl + 8);
     memcpy(J.band_start, g_na_band, sizeof J.band_start);
     launch_decode_lists(J, sms, st);
@@ -152,14 +156,18 @@ VC_API int vcg_decode_atoms_noalloc(const uint8_t *payload_dev, size_t payload_b
         vcd_set_error("no-alloc decode: kernel launch", e);
         return 4;
     }
-    uint32_t err = 0xFFFFFFFFu;
-    e = cudaMemcpyAsync(&err, base + kNaCtl, 4, cudaMemcpyDeviceToHost, st);
+    uint32_t err[2] = {0xFFFFFFFFu, 0};   // [first malformed atom][a wait ran out]
+    e = cudaMemcpyAsync(err, base + kNaCtl, 8, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         vcd_set_error("no-alloc decode", e);
         return 4;
     }
-    if (err < n_atoms) {
+    if (err[1]) {
+        vcd_set_error("no-alloc decode: a wait inside a kernel ran out", cudaSuccess);
+        return 4;
+    }
+    if (err[0] < n_atoms) {
         vcd_set_error("no-alloc decode: malformed payload", cudaSuccess);
         return 1;
     }
