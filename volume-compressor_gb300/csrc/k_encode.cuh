@@ -60,21 +60,29 @@ struct FwdJob {
     int coef_store;
 };
 
+// Coder pass over the lists of n_atoms atoms.
 struct RcJob {
     uint64_t n_atoms;
     const uint32_t *meta;
     const uint32_t *ent;
     uint32_t band_start[9];
-    // size pass
     uint32_t *len;                       // payload bytes per atom ([dc] + coder bytes; 0 = zero atom)
-    unsigned long long *total_bytes;
+    uint32_t *sums;                      // optional: kSums words per atom, what k_resolve makes the bytes of
+    unsigned long long *total_bytes;     // optional: added up over the atoms
     unsigned long long *total_present;
-    // write pass
+};
+
+// Payloads from the sums of a coder pass.
+struct ResolveJob {
+    uint64_t n_atoms;
+    const uint32_t *meta;
+    const uint32_t *ent;                 // the lists, for atoms with too many sums for their slot
+    uint32_t band_start[9];
+    const uint32_t *len;
+    const uint32_t *sums;                // null: code every atom from its list
     uint8_t *arc;
     const uint64_t *dst_off;             // optional: per atom (this launch) payload offset in arc
-    uint64_t slot_bytes;                 // optional: atom t's payload at arc + t * slot_bytes, at most that long
-                                         // (len[t] receives the full length, stored or not)
-    const uint64_t *pos;                 // canonical exclusive scan of consumed bytes
+    const uint64_t *pos;                 // else: canonical exclusive scan of consumed bytes
     uint64_t canon_first;                // canonical index of this chunk's first atom
     Layout lay;
 };
@@ -91,12 +99,11 @@ struct PlaceJob {
 void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s);
 // atoms that are all LOD0 with kept coefficients: quantise and compact only
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s);
-void launch_rc_encode(const RcJob &J, bool write, int num_sms, cudaStream_t s);
+// lengths, and the sums where J.sums is set
+void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s);
+void launch_resolve(const ResolveJob &J, cudaStream_t s);
 void launch_consume(const PlaceJob &J, cudaStream_t s);
 void launch_slots(const PlaceJob &J, cudaStream_t s);
 void launch_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, cudaStream_t s);
-// payloads of n atoms from fixed slots (slot bytes apart) to packed offsets
-void launch_pack(const uint8_t *slots, uint64_t slot, const uint32_t *len, const uint64_t *off, uint64_t n,
-                 uint8_t *dst, cudaStream_t s);
 
 }  // namespace vcg

@@ -11,6 +11,7 @@
 #include "k_ds.cuh"
 #include "k_encode.cuh"
 #include "kernels.cuh"
+#include "rc_encode.cuh"
 #include "vc_device.h"
 
 using namespace vcg;
@@ -34,7 +35,10 @@ struct EncState {
     Layout lay;
     const uint8_t *lvol[8];
     uint32_t dims[8][3];
-    uint32_t *ent, *meta, *len, *best;
+    uint32_t *ent, *meta, *len, *best;   // lists and meta: LOD0's, or a chunk's
+    uint32_t *ent2, *meta2;              // the coarser LODs', beside them (null: none)
+    uint32_t *sums;                      // the coder's sums, kSums words an atom
+    bool whole;                          // lists and sums of every atom are kept: one coder pass
     uint64_t *pos;
     uint8_t *dc, *arc;
     unsigned long long *red;
@@ -53,94 +57,150 @@ static void set_q(EncState &S, int lod, float q) {
     cudaMemcpyAsync(S.qtab + lod, &S.qh, sizeof(vcd_quant), cudaMemcpyHostToDevice, S.c->stream);
 }
 
+enum EncPass { kSizes, kCode, kWrite };
+
 // Forward + coder passes over canonical atoms [a0, a1) (any mix of LODs, each at
 // the q in the device table) on stream st with list and metadata scratch ent,
-// meta (kChunk atoms): size-only (lengths into len and the totals) or writing
-// payloads into the archive. One launch pair per kChunk atoms: a coder launch
-// costs about one atom's serial coding time however many atoms it holds.
-static int run_range(EncState &S, uint64_t a0, uint64_t a1, bool write, cudaStream_t st, uint32_t *ent,
-                     uint32_t *meta) {
-    for (uint64_t c0 = a0; c0 < a1; c0 += kChunk) {
-        const uint64_t n = a1 - c0 < kChunk ? a1 - c0 : kChunk;
-        FwdJob F;
-        memset(&F, 0, sizeof F);   // fields this pass does not use stay null
-        F.lay = S.lay;
-        memcpy(F.vol, S.lvol, sizeof F.vol);
-        memcpy(F.dims, S.dims, sizeof F.dims);
-        F.first = c0;
-        F.n_atoms = n;
-        F.q = S.qtab;
-        F.scan = g_dev.tables->scan;
-        F.alt_mask = g_dev.tables->alt_mask;
-        F.ent = ent;
-        F.meta = meta;
-        F.coef = S.coef;
-        F.coef_dc = S.coef_dc;
-        F.coef_n = S.coef_n;
-        F.coef_store = !S.coef_valid;
-        const bool from_cache = S.coef && S.coef_valid && c0 + n <= S.coef_n;
-        const bool prof = vcd_prof_on();
-        if (prof) cudaEventRecord(S.c->ev[4], st);
-        if (from_cache) launch_quant_cached(F, g_dev.num_sms, st);
-        else launch_fwd(F, g_dev.num_sms, st);
-        RcJob R;
-        memset(&R, 0, sizeof R);
-        R.n_atoms = n;
-        R.meta = meta;
-        R.ent = ent;
-        memcpy(R.band_start, g_dev.band_start, sizeof R.band_start);
-        if (!write) {
-            R.len = S.len + c0;
-            R.total_bytes = S.red;
-            R.total_present = S.red + 1;
-        } else {
-            R.arc = S.arc;
-            R.pos = S.pos;
-            R.canon_first = c0;
-            R.lay = S.lay;
-            launch_gather_dc(meta, n, S.dc + c0, st);
-        }
-        if (prof) cudaEventRecord(S.c->ev[5], st);
-        launch_rc_encode(R, write, g_dev.num_sms, st);
-        if (S.coef && c0 < S.coef_n && c0 + n >= S.coef_n) S.coef_valid = true;   // LOD0 transform kept
-        if (prof) {
-            cudaEventRecord(S.c->ev[1], st);
-            cudaEventSynchronize(S.c->ev[1]);
-            // forward: volume bytes in (the lists it writes are scratch, not counted)
-            if (from_cache)   // coefficients in, lists out (scratch, not counted)
-                vcd_prof_add("quant_cached", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * 131072ull, 0, n);
-            else
-                vcd_prof_add("fwd_dct_quant", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * 32768ull, 0, n);
-            vcd_prof_add(write ? "rc_encode_write" : "rc_encode_size", vcd_elapsed(S.c->ev[5], S.c->ev[1]), 1, 0,
-                         0, n);
-        }
+// meta (kChunk atoms). kSizes: lengths into len and the totals. kCode: lengths,
+// and the sums (of canonical atom a at slot a) for a resolve once the payloads'
+// places are known. kWrite: sums, a chunk's at a time, and payloads into the
+// archive. One launch pair per kChunk atoms: a coder launch costs about one
+// atom's serial coding time however many atoms it holds.
+static void resolve_range(EncState &S, uint64_t c0, uint64_t n, const uint32_t *ent, const uint32_t *meta,
+                          const uint32_t *sums, cudaStream_t st) {
+    ResolveJob W;
+    memset(&W, 0, sizeof W);
+    W.n_atoms = n;
+    W.meta = meta;
+    W.ent = ent;
+    memcpy(W.band_start, g_dev.band_start, sizeof W.band_start);
+    W.len = S.len + c0;
+    W.sums = sums;
+    W.arc = S.arc;
+    W.pos = S.pos;
+    W.canon_first = c0;
+    W.lay = S.lay;
+    const bool prof = vcd_prof_on();
+    if (prof) cudaEventRecord(S.c->ev[5], st);
+    launch_resolve(W, st);
+    if (prof) {
+        cudaEventRecord(S.c->ev[1], st);
+        cudaEventSynchronize(S.c->ev[1]);
+        vcd_prof_add("encode_resolve", vcd_elapsed(S.c->ev[5], S.c->ev[1]), 1, 0, 0, n);
     }
-    return 0;
 }
 
-// The same over [0, total): LOD0 on the context's stream and the coarser LODs
+// forward pass over canonical atoms [c0, c0 + n)
+static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uint32_t *ent, uint32_t *meta) {
+    FwdJob F;
+    memset(&F, 0, sizeof F);   // fields this pass does not use stay null
+    F.lay = S.lay;
+    memcpy(F.vol, S.lvol, sizeof F.vol);
+    memcpy(F.dims, S.dims, sizeof F.dims);
+    F.first = c0;
+    F.n_atoms = n;
+    F.q = S.qtab;
+    F.scan = g_dev.tables->scan;
+    F.alt_mask = g_dev.tables->alt_mask;
+    F.ent = ent;
+    F.meta = meta;
+    F.coef = S.coef;
+    F.coef_dc = S.coef_dc;
+    F.coef_n = S.coef_n;
+    F.coef_store = !S.coef_valid;
+    const bool from_cache = S.coef && S.coef_valid && c0 + n <= S.coef_n;
+    const bool prof = vcd_prof_on();
+    if (prof) cudaEventRecord(S.c->ev[4], st);
+    if (from_cache) launch_quant_cached(F, g_dev.num_sms, st);
+    else launch_fwd(F, g_dev.num_sms, st);
+    if (S.coef && c0 < S.coef_n && c0 + n >= S.coef_n) S.coef_valid = true;   // LOD0 transform kept
+    if (prof) {
+        cudaEventRecord(S.c->ev[5], st);
+        cudaEventSynchronize(S.c->ev[5]);
+        // forward: volume bytes in (the lists it writes are scratch, not counted)
+        if (from_cache)   // coefficients in, lists out (scratch, not counted)
+            vcd_prof_add("quant_cached", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * 131072ull, 0, n);
+        else
+            vcd_prof_add("fwd_dct_quant", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * 32768ull, 0, n);
+    }
+}
+
+// coder pass over the lists of canonical atoms [c0, c0 + n)
+static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaStream_t st, uint32_t *ent,
+                       uint32_t *meta, uint32_t *sums) {
+    RcJob R;
+    memset(&R, 0, sizeof R);
+    R.n_atoms = n;
+    R.meta = meta;
+    R.ent = ent;
+    memcpy(R.band_start, g_dev.band_start, sizeof R.band_start);
+    R.len = S.len + c0;
+    if (pass == kSizes) {
+        R.total_bytes = S.red;
+        R.total_present = S.red + 1;
+    } else {
+        // without room for sums the payloads are coded from the lists (kWrite)
+        R.sums = pass == kCode ? sums + c0 * kSums : sums;
+        launch_gather_dc(meta, n, S.dc + c0, st);
+    }
+    const bool prof = vcd_prof_on();
+    if (prof) cudaEventRecord(S.c->ev[5], st);
+    if (pass == kSizes || R.sums) launch_rc_encode(R, g_dev.num_sms, st);
+    if (prof) {
+        cudaEventRecord(S.c->ev[1], st);
+        cudaEventSynchronize(S.c->ev[1]);
+        vcd_prof_add(pass == kSizes ? "rc_encode_size" : "rc_encode_write", vcd_elapsed(S.c->ev[5], S.c->ev[1]), 1, 0,
+                     0, n);
+    }
+    if (pass == kWrite) resolve_range(S, c0, n, ent, meta, R.sums, st);
+}
+
+static void run_range(EncState &S, uint64_t a0, uint64_t a1, EncPass pass, cudaStream_t st, uint32_t *ent,
+                      uint32_t *meta, uint32_t *sums = nullptr) {
+    for (uint64_t c0 = a0; c0 < a1; c0 += kChunk) {
+        const uint64_t n = a1 - c0 < kChunk ? a1 - c0 : kChunk;
+        fwd_chunk(S, c0, n, st, ent, meta);
+        code_chunk(S, c0, n, pass, st, ent, meta, sums);
+    }
+}
+
+// The same over all atoms: LOD0 on the context's stream and the coarser LODs
 // beside it on the second stream, with their own list scratch. The coarser LODs
 // are few atoms but the finest-quantised ones (q down to 0.05): one of them is a
 // serial coder chain longer than a whole LOD0 pass, so run after LOD0 it would
 // add its length. Serial under per-stage measurement (its events are per stream).
-static int run_split(EncState &S, uint64_t na0, uint64_t total, bool write) {
+static void run_split(EncState &S, uint64_t na0, uint64_t total, uint64_t chunk, EncPass pass) {
     vcd_ctx *c = S.c;
-    cudaStream_t side = (total > na0 && na0 && !vcd_prof_on()) ? vcd_side_stream(c) : NULL;
-    void *pe = NULL, *pm = NULL;
-    const uint64_t n1 = total - na0 < kChunk ? total - na0 : kChunk;
-    if (side && (vcd_scratch(c, VCD_BUF_EENT2, n1 * VCD_MAX_ENTRIES * 4 + 16, &pe) != cudaSuccess ||
-                 vcd_scratch(c, VCD_BUF_EMETA2, n1 * 4 + 16, &pm) != cudaSuccess)) {
-        cudaGetLastError();
-        side = NULL;
+    // chunks of a kWrite have their own sums on each stream
+    uint32_t *sums2 = pass == kWrite && S.sums ? S.sums + chunk * kSums : S.sums;
+    if (!S.ent2) {
+        run_range(S, 0, total, pass, c->stream, S.ent, S.meta, S.sums);
+        return;
     }
-    if (!side) return run_range(S, 0, total, write, c->stream, S.ent, S.meta);
-    cudaEventRecord(c->chunk_ev[0], c->stream);   // the side stream starts after the work queued so far
-    cudaStreamWaitEvent(side, c->chunk_ev[0], 0);
-    run_range(S, na0, total, write, side, (uint32_t *)pe, (uint32_t *)pm);
-    run_range(S, 0, na0, write, c->stream, S.ent, S.meta);
-    cudaEventRecord(c->chunk_ev[1], side);
-    cudaStreamWaitEvent(c->stream, c->chunk_ev[1], 0);
-    return 0;
+    cudaStream_t side = vcd_prof_on() ? NULL : vcd_side_stream(c), st1 = side ? side : c->stream;
+    // A forward CTA takes nearly all shared memory of an SM, so beside a coder it
+    // waits for the coder's CTAs: where one chunk holds each range, both forward
+    // passes go first and only the coders run side by side.
+    const bool first = total - na0 <= kChunk && na0 <= kChunk;
+    if (first) {
+        fwd_chunk(S, na0, total - na0, c->stream, S.ent2, S.meta2);
+        fwd_chunk(S, 0, na0, c->stream, S.ent, S.meta);
+    }
+    if (side) {
+        cudaEventRecord(c->chunk_ev[0], c->stream);   // the side stream starts after the work queued so far
+        cudaStreamWaitEvent(side, c->chunk_ev[0], 0);
+    }
+    if (first) {
+        code_chunk(S, na0, total - na0, pass, st1, S.ent2, S.meta2, sums2);
+        code_chunk(S, 0, na0, pass, c->stream, S.ent, S.meta, S.sums);
+    } else {
+        run_range(S, na0, total, pass, st1, S.ent2, S.meta2, sums2);
+        run_range(S, 0, na0, pass, c->stream, S.ent, S.meta, S.sums);
+    }
+    if (side) {
+        cudaEventRecord(c->chunk_ev[1], side);
+        cudaStreamWaitEvent(c->stream, c->chunk_ev[1], 0);
+    }
 }
 
 extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info, uint8_t **out, size_t *out_len) {
@@ -221,6 +281,27 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         }
         cudaGetLastError();
     }
+    {   // One coder pass for all where the lists and sums of every atom have room (256 KiB an atom, the sums
+        // in at most half the free memory): else one for the sizes and one, a chunk at a time, for the bytes.
+        size_t fr = 0, tot = 0;
+        const uint64_t n1 = total_atoms - na0, n1c = n1 < kChunk ? n1 : kChunk;
+        const size_t all_b = (size_t)total_atoms * kSums * 4;
+        void *pe = NULL, *pm = NULL;
+        if (n1 && vcd_scratch(c, VCD_BUF_EENT2, n1c * VCD_MAX_ENTRIES * 4 + 16, &pe) == cudaSuccess &&
+            vcd_scratch(c, VCD_BUF_EMETA2, n1c * 4 + 16, &pm) == cudaSuccess) {
+            S.ent2 = (uint32_t *)pe;
+            S.meta2 = (uint32_t *)pm;
+        }
+        if (na0 <= kChunk && n1 <= kChunk && (S.ent2 || !n1) && cudaMemGetInfo(&fr, &tot) == cudaSuccess &&
+            (c->cap[VCD_BUF_ESUM] >= all_b || all_b <= fr / 2) &&
+            vcd_scratch(c, VCD_BUF_ESUM, all_b, &p) == cudaSuccess) {
+            S.whole = true;
+            S.sums = (uint32_t *)p;
+        } else if (vcd_scratch(c, VCD_BUF_ESUM, (size_t)(chunk + (S.ent2 ? n1c : 0)) * kSums * 4, &p) == cudaSuccess) {
+            S.sums = (uint32_t *)p;
+        }
+        cudaGetLastError();
+    }
 
     // ---- rate control on LOD0 (bisection over float bit patterns of [0.05, 4096])
     uint32_t lo = b_of(0.05f), hi = b_of(4096.0f);
@@ -233,7 +314,7 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         float q = f_of(mid);
         CK(cudaMemsetAsync(S.red, 0, 16, st), "totals reset");
         set_q(S, 0, q);
-        run_range(S, 0, na0, false, st, S.ent, S.meta);
+        run_range(S, 0, na0, kSizes, st, S.ent, S.meta);
         unsigned long long h[2];
         CK(cudaMemcpyAsync(h, S.red, 16, cudaMemcpyDeviceToHost, st), "totals read");
         CK(cudaStreamSynchronize(st), "rate control pass");
@@ -246,7 +327,7 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
             best_q = q;
             best_bytes = h[0];
             have_best = true;
-            CK(cudaMemcpyAsync(S.best, S.len, na0 * 4, cudaMemcpyDeviceToDevice, st), "keep sizes");
+            if (!S.whole) CK(cudaMemcpyAsync(S.best, S.len, na0 * 4, cudaMemcpyDeviceToDevice, st), "keep sizes");
         }
         if (ratio < (double)info->target_ratio) lo = mid; else hi = mid;
     }
@@ -262,14 +343,16 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         for (int l = 0; l < nlod; ++l) { qs[l] = vch_clamp_q(q < 0.05f ? 0.05f : q); q = q * 0.6f; }
     }
 
-    // ---- sizes of every atom at its LOD's q (LODs 1.. together in one pass)
+    // ---- every atom at its LOD's q: coded, or its size (LODs 1.. together in one pass)
     for (int l = 0; l < nlod; ++l) set_q(S, l, qs[l]);
-    if (have_best) {
+    if (S.whole) {
+        run_split(S, na0, total_atoms, chunk, kCode);
+    } else if (have_best) {
         CK(cudaMemcpyAsync(S.len, S.best, na0 * 4, cudaMemcpyDeviceToDevice, st), "restore sizes");
-        run_range(S, na0, total_atoms, false, st, S.ent, S.meta);
+        run_range(S, na0, total_atoms, kSizes, st, S.ent, S.meta);
     } else {
         CK(cudaMemsetAsync(S.red, 0, 16, st), "totals reset");
-        run_split(S, na0, total_atoms, false);
+        run_split(S, na0, total_atoms, chunk, kSizes);
     }
 
     // ---- canonical placement: exclusive scan of consumed bytes
@@ -302,7 +385,12 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     S.arc = (uint8_t *)p;
     P.arc = S.arc;
     cudaMemsetAsync(S.arc, 0, total, st);
-    run_split(S, na0, total_atoms, true);
+    if (S.whole) {
+        resolve_range(S, 0, na0, S.ent, S.meta, S.sums, st);
+        if (S.ent2) resolve_range(S, na0, total_atoms - na0, S.ent2, S.meta2, S.sums + na0 * kSums, st);
+    } else {
+        run_split(S, na0, total_atoms, chunk, kWrite);
+    }
     if (prof) cudaEventRecord(c->ev[4], st);
     launch_slots(P, st);
     if (prof) {   // one 16-byte slot per atom
@@ -350,12 +438,13 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     free(hd);
     if (e != cudaSuccess) { free(res); vcd_set_error("archive assembly", e); return vcd_status_of(e); }
     c->last_ms = vcd_elapsed(c->ev[6], c->ev[7]);
-    {   // a large transform cache is not kept between encodes (more than 1/8 of the device memory)
+    // a large transform cache or sums are not kept between encodes (more than 1/8 of the device memory)
+    for (int b : {(int)VCD_BUF_COEF, (int)VCD_BUF_ESUM}) {
         size_t fr = 0, tot = 0;
-        if (c->buf[VCD_BUF_COEF] && cudaMemGetInfo(&fr, &tot) == cudaSuccess && c->cap[VCD_BUF_COEF] > tot / 8) {
-            cudaFree(c->buf[VCD_BUF_COEF]);
-            c->buf[VCD_BUF_COEF] = NULL;
-            c->cap[VCD_BUF_COEF] = 0;
+        if (c->buf[b] && cudaMemGetInfo(&fr, &tot) == cudaSuccess && c->cap[b] > tot / 8) {
+            cudaFree(c->buf[b]);
+            c->buf[b] = NULL;
+            c->cap[b] = 0;
         }
         cudaGetLastError();
     }
@@ -367,15 +456,10 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
 // ---------------------------------------------------------------- writer batches
 // Independent atoms (box rasters or stacked single atoms) through the same
 // forward and coder kernels as the whole-volume encoder, with one coder pass:
-// per chunk of at most kWChunk atoms a forward pass and a writing coder pass
-// into fixed slots of kSlot bytes (the reference encoder's largest atom:
-// 1 + 4 * 32768 + 64 bytes, rounded up), the lengths back to the host for the
-// packing offsets, and a packing kernel whose output is copied into the
-// thread's pinned buffer. An atom longer than its slot (where the reference's
-// encoder stops with "range encoder overflow") makes its chunk take a second,
-// exact writing pass.
+// per chunk of at most kWChunk atoms a forward pass and a coder pass, the lengths
+// back to the host for the packing offsets, and a resolve into the packed buffer,
+// which is copied into the thread's pinned buffer.
 static const uint64_t kWChunk = 8192;
-static const uint64_t kSlot = 131200;
 
 extern "C" int vcd_encode_segments(const vcd_seg *segs, int nseg, const float *qs, int nq, uint8_t **pay,
                                    uint64_t *pay_bytes) {
@@ -429,41 +513,39 @@ extern "C" int vcd_encode_segments(const vcd_seg *segs, int nseg, const float *q
             F.ent = ent;
             F.meta = dmeta;
             launch_fwd(F, g_dev.num_sms, st);
-            if ((e = vcd_scratch(c, VCD_BUF_ARC, n * kSlot + 16, &p)) != cudaSuccess) break;
-            uint8_t *dslots = (uint8_t *)p;
-            RcJob W;
-            memset(&W, 0, sizeof W);
-            W.n_atoms = n;
-            W.meta = dmeta;
-            W.ent = ent;
-            memcpy(W.band_start, g_dev.band_start, sizeof W.band_start);
-            W.arc = dslots;
-            W.slot_bytes = kSlot;
-            W.len = dlen;
-            launch_rc_encode(W, true, g_dev.num_sms, st);
+            if ((e = vcd_scratch(c, VCD_BUF_ESUM, n * kSums * 4, &p)) != cudaSuccess) break;
+            RcJob R;
+            memset(&R, 0, sizeof R);
+            R.n_atoms = n;
+            R.meta = dmeta;
+            R.ent = ent;
+            memcpy(R.band_start, g_dev.band_start, sizeof R.band_start);
+            R.len = dlen;
+            R.sums = (uint32_t *)p;
+            launch_rc_encode(R, g_dev.num_sms, st);
             if ((e = cudaMemcpyAsync(S.len + c0, dlen, n * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
                 (e = cudaStreamSynchronize(st)) != cudaSuccess)
                 break;
             uint64_t bytes = 0;
-            bool over = false;
             for (uint64_t i = 0; i < n; ++i) {
                 offh[i] = bytes;
                 S.off[c0 + i] = total + bytes;
                 bytes += S.len[c0 + i];
-                over |= S.len[c0 + i] > kSlot;
             }
             if ((e = vcd_scratch(c, VCD_BUF_WPACK, bytes + 16, &p)) != cudaSuccess) break;
             uint8_t *dpack = (uint8_t *)p;
             if ((e = cudaMemcpyAsync(doff, offh, n * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-            if (!over) {
-                launch_pack(dslots, kSlot, dlen, doff, n, dpack, st);
-            } else {   // exact second pass for a chunk with an atom longer than its slot
-                W.slot_bytes = 0;
-                W.len = nullptr;
-                W.arc = dpack;
-                W.dst_off = doff;
-                launch_rc_encode(W, true, g_dev.num_sms, st);
-            }
+            ResolveJob W;
+            memset(&W, 0, sizeof W);
+            W.n_atoms = n;
+            W.meta = dmeta;
+            W.ent = ent;
+            memcpy(W.band_start, R.band_start, sizeof W.band_start);
+            W.len = dlen;
+            W.sums = R.sums;
+            W.arc = dpack;
+            W.dst_off = doff;
+            launch_resolve(W, st);
             if (total + bytes > c->wpin_cap) {   // grow the pinned output, keeping what it holds
                 if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
                 size_t want = (total + bytes) + (total + bytes) / 2 + (1 << 20);
