@@ -13,7 +13,9 @@
 //                 order (an L2 block of 512 KiB at a region's first atom, then the
 //                 payload) and the 16-byte L2 slots (src/vc/vc.c:1082-1159)
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "dct32.cuh"
 #include "k_encode.cuh"
@@ -282,6 +284,8 @@ __global__ void __launch_bounds__(kFwdThreads) k_quant_cached(FwdJob J) {
     }
 }
 
+constexpr size_t size_smem(int A) { return sizeof(EncCosts) + 8 * (size_t)A * kRingPitch * 4; }
+
 // Atom t's list, or none; whether it is present (its dc is coded).
 __device__ __forceinline__ bool enc_atom(const RcJob &J, uint64_t t, const uint32_t *&ent, uint32_t &nnz) {
     const uint32_t meta = t < J.n_atoms ? J.meta[t] : kMetaZero;
@@ -291,21 +295,9 @@ __device__ __forceinline__ bool enc_atom(const RcJob &J, uint64_t t, const uint3
     return on;
 }
 
-// n coder bytes of atom t (every lane of the warp; t < n_atoms only where the lane holds one)
-__device__ __forceinline__ void enc_count(const RcJob &J, uint64_t t, bool on, uint32_t n) {
-    if (t < J.n_atoms) J.len[t] = on ? n + 1u : 0u;
-    if (!J.total_bytes) return;
-    const unsigned long long b = on ? n + 1u : 0u;
-    const uint32_t present = __popc(__ballot_sync(0xFFFFFFFFu, on));
-    const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)b);   // 32 lanes of at most 2^18 bytes
-    if ((threadIdx.x & 31u) == 0u && present) {
-        atomicAdd(J.total_bytes, (unsigned long long)sum);
-        atomicAdd(J.total_present, (unsigned long long)present);
-    }
-}
-
 // Few atoms: kEncGroups groups of G atoms per CTA. Warps 0..3 code, the warps
-// after them produce, warp w for group w % 4 (the same SM sub-partition).
+// after them produce, warp w for group w % 4 (the same SM sub-partition). Without
+// SUMS: the lengths of the atoms in doubt, G = 1.
 template <bool SUMS>
 __global__ void __launch_bounds__(32 * kEncGroups * enc_group_warps(kGroupMax)) k_rc_encode_groups(RcJob J, uint32_t G) {
     extern __shared__ __align__(16) uint8_t gmem[];
@@ -315,25 +307,90 @@ __global__ void __launch_bounds__(32 * kEncGroups * enc_group_warps(kGroupMax)) 
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, c = warp % kEncGroups, w = warp / kEncGroups;
     EncGroup g;
     g.init(gmem + c * enc_group_bytes(G), G, 1u + c);
-    const uint64_t t0 = ((uint64_t)blockIdx.x * kEncGroups + c) * G;
-    const uint32_t *ent;
-    uint32_t nnz;
-    if (w == 0u) {
-        const uint64_t t = lane < G ? t0 + lane : J.n_atoms;
+    const uint64_t n = SUMS ? J.n_atoms : J.doubt[0];
+    for (uint64_t b = blockIdx.x; b * kEncGroups * G < n; b += gridDim.x) {
+        const uint64_t t0 = (b * kEncGroups + c) * G;
+        const uint32_t slot = w == 0u ? lane : (enc_group_split(G) ? 0u : 2u * (w - 1u)) + (lane >> 4);
+        uint64_t t = slot < G ? t0 + slot : n;
+        t = t >= n ? J.n_atoms : SUMS ? t : J.doubt[1u + t];
+        const uint32_t *ent;
+        uint32_t nnz;
         const bool on = enc_atom(J, t, ent, nnz);
-        const uint32_t eob = nnz ? (ent[nnz - 1u] & 0xFFFFu) + 1u : 0u;
-        const uint32_t n = enc_consume<SUMS>(g, on, eob, SUMS ? J.sums + (on ? t : 0) * kSums : nullptr, lane);
-        enc_count(J, t, on, n);
-    } else {
-        const bool split = enc_group_split(G);
-        const uint32_t slot = (split ? 0u : 2u * (w - 1u)) + (lane >> 4);
-        enc_atom(J, slot < G ? t0 + slot : J.n_atoms, ent, nnz);
-        enc_produce(g, slot, ent, nnz, bstart, lane, !split || w == 1u, !split || w == 2u);
+        if (w == 0u) {
+            const uint32_t eob = nnz ? (ent[nnz - 1u] & 0xFFFFu) + 1u : 0u;
+            const uint32_t k = enc_consume<SUMS>(g, on, eob, SUMS ? J.sums + (on ? t : 0) * kSums : nullptr, lane);
+            if (t < J.n_atoms) {
+                if (!SUMS && on) atomicAdd(J.totals, (unsigned long long)(k + 1u - J.len[t]));
+                J.len[t] = on ? k + 1u : 0u;
+            }
+        } else {
+            const bool split = enc_group_split(G);
+            enc_produce(g, slot, ent, nnz, bstart, lane, !split || w == 1u, !split || w == 2u);
+        }
+        g.sync();   // the counts are the next atoms'
+    }
+}
+
+// Lengths alone: A atoms at a time, A / 4 warps their bands (as many atoms a warp
+// as A, so with 32 of them a warp's bands are alike), A / 2 warps the unary
+// contexts of two each; those that the costs leave in doubt are collected for
+// the coder. A pass over 540 atoms of 30,000 decisions takes 0.25 ms (A 4; the
+// coder 1.14 ms), one over 32,768 of 48,700 takes 4.3 ms (A 32; a coder's lane each 5.7, the lockstep coder 9.3).
+template <int A>
+__global__ void __launch_bounds__(24 * A) k_rc_sizes(RcJob J) {
+    extern __shared__ __align__(16) uint8_t gmem[];
+    EncCosts &T = *reinterpret_cast<EncCosts *>(gmem);
+    uint32_t *ring = reinterpret_cast<uint32_t *>(gmem + sizeof(EncCosts));
+    __shared__ uint32_t bstart[9];
+    __shared__ unsigned long long cost[A];
+    __shared__ uint32_t lo[A], hi[A];
+    const uint32_t tid = threadIdx.x;
+    if (tid < 9) bstart[tid] = J.band_start[tid];
+    for (uint32_t i = tid; i < sizeof(EncCosts) / 16; i += blockDim.x)
+        reinterpret_cast<uint4 *>(gmem)[i] = __ldg(reinterpret_cast<const uint4 *>(J.costs) + i);
+    const uint32_t lane = tid & 31u, warp = tid >> 5;
+    const bool bands = warp < A / 4;
+    const uint32_t b = A == 4 ? lane & 7u : warp;   // the lane's band
+    const uint32_t a = !bands ? 2u * (warp - A / 4) + (lane >> 4) : A == 4 ? lane >> 3 : lane;
+    for (uint64_t t0 = (uint64_t)blockIdx.x * A; t0 < J.n_atoms; t0 += (uint64_t)gridDim.x * A) {
+        if (tid < A) cost[tid] = 0, lo[tid] = 0, hi[tid] = 0;
+        __syncthreads();
+        const uint32_t *ent;
+        uint32_t nnz;
+        enc_atom(J, t0 + a, ent, nnz);
+        const EncSize r = bands ? enc_size_bands<A == 4>(T, ent, nnz, b, bstart, ring + tid * kRingPitch)
+                                : enc_size_rest(T, ent, nnz, lane);
+        atomicAdd(&cost[a], (unsigned long long)r.cost);
+        atomicAdd(&lo[a], r.lo);
+        atomicAdd(&hi[a], r.hi);
+        __syncthreads();
+        if (tid < 32u) {
+            const uint64_t t = tid < A ? t0 + tid : J.n_atoms;
+            const uint32_t m = t < J.n_atoms ? J.meta[t] : kMetaZero;
+            const bool on = !(m & kMetaZero);
+            const uint32_t i = tid % A;
+            // the end of the list is 16 bypass decisions; an interval of 2^32 - 1
+            // to start with costs less than one unit
+            const uint64_t least = 16ull * kCostOne + cost[i] - lo[i];
+            const uint64_t most = 16ull * kCostOne + cost[i] + hi[i] + 16u * kCostBypass + 1u;
+            uint32_t n = (uint32_t)((least - 1u) / (8ull * kCostOne));
+            bool sure = most < (n + 1ull) * 8ull * kCostOne;
+            if (!(m & 0xFFFFu)) n = 2u, sure = true;   // 16 halvings of 2^32 - 1
+            if (t < J.n_atoms) J.len[t] = on ? n + 6u : 0u;
+            if (on && !sure) J.doubt[1u + atomicAdd(J.doubt, 1u)] = (uint32_t)t;
+            const uint32_t bytes = __reduce_add_sync(0xFFFFFFFFu, on ? n + 6u : 0u);
+            const uint32_t present = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, on));
+            const uint32_t doubt = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, on && !sure));
+            if (tid == 0u && present) {
+                atomicAdd(J.totals, (unsigned long long)bytes);
+                atomicAdd(J.totals + 1, (unsigned long long)present);
+                if (doubt) atomicAdd(J.totals + 2, (unsigned long long)doubt);
+            }
+        }
     }
 }
 
 // Many atoms: a lane each, G per warp.
-template <bool SUMS>
 __global__ void __launch_bounds__(128) k_rc_encode_lanes(RcJob J, uint32_t G) {
     __shared__ uint32_t bstart[9];
     __shared__ __align__(16) uint32_t mem[4][kEncWarpWords];
@@ -344,9 +401,8 @@ __global__ void __launch_bounds__(128) k_rc_encode_lanes(RcJob J, uint32_t G) {
     const uint32_t *ent;
     uint32_t nnz;
     const bool on = enc_atom(J, t, ent, nnz);
-    const uint32_t n = enc_lanes<SUMS, 4, 3, 2>(on, ent, nnz, bstart, SUMS ? J.sums + (on ? t : 0) * kSums : nullptr,
-                                                mem[warp], lane);
-    enc_count(J, t, on, n);
+    const uint32_t n = enc_lanes<4, 3, 2>(on, ent, nnz, bstart, J.sums + (on ? t : 0) * kSums, mem[warp], lane);
+    if (t < J.n_atoms) J.len[t] = on ? n + 1u : 0u;
 }
 
 // A warp per atom: [dc] and the coder bytes.
@@ -415,7 +471,8 @@ void enc_set_smem() {
     smem_attr((const void *)k_fwd, (int)kFwdSmem);
     smem_attr((const void *)k_quant_cached, (int)kQuantSmem);
     smem_attr((const void *)k_rc_encode_groups<true>, (int)(kEncGroups * enc_group_bytes(kGroupMax)));
-    smem_attr((const void *)k_rc_encode_groups<false>, (int)(kEncGroups * enc_group_bytes(kGroupMax)));
+    smem_attr((const void *)k_rc_sizes<4>, (int)size_smem(4));
+    smem_attr((const void *)k_rc_sizes<32>, (int)size_smem(32));
 }
 
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s) {
@@ -432,29 +489,65 @@ void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s) {
     k_fwd<<<(unsigned)grid, kFwdThreads, kFwdSmem, s>>>(J);
 }
 
-// Up to kGroupMax atoms per SM sub-partition (4,864 on 152 SMs) run as groups,
-// one coder warp per sub-partition; more of them a lane each, with the fewest
-// warps per sub-partition that hold them at 32 a warp, spread evenly. At the
-// line: 4,681 atoms of 30,000 decisions in 2.6 ms as groups of 8 and 3.2 ms a lane
-// each, of 164,000 decisions in 9.6 and 21.6 ms.
+void enc_costs(EncCosts *t) {
+    memset(t, 0, sizeof *t);
+    const double bit = kCostOne, e = 4096.0 / 16777216.0 * 1.4427 * 1.0001;   // log2(e) and the square term, above
+    for (uint32_t c = 1; c < 4096; ++c)
+        t->one[c] = make_uint2((uint32_t)llround((12.0 - log2((double)c)) * bit),
+                               (uint32_t)ceil(e * bit / c) + kCostSlack);
+    for (uint32_t q0 = 1; q0 < 4096; ++q0) {
+        uint32_t q = q0;
+        double cost = 0.0, err = 0.0;
+        for (int j = 0; j < 8; ++j) {
+            const double c = 4096.0 - q;
+            cost += 12.0 - log2(c);
+            err += e * bit / c;
+            q -= q >> 5;
+        }
+        t->eight[q0] = make_uint2((uint32_t)llround(fmin(cost * bit, 4294967295.0)),
+                                  (uint32_t)fmin(ceil(err) + kCostSlack, 65535.0) << 16 | q);
+    }
+}
+
+// Lengths alone come from costs (three CTAs of 4 atoms an SM while that holds
+// them all, else two of 32), and where they have to be exact the atoms in doubt,
+// one in a thousand, are then coded. With sums, up to kGroupMax atoms per SM
+// sub-partition (4,864 on 152 SMs) run as groups, one coder warp per
+// sub-partition; more of them a lane each, with the fewest warps per
+// sub-partition that hold them at 32 a warp, spread evenly. At the line: 4,681
+// atoms of 30,000 decisions in 2.6 ms as groups of 8 and 3.2 ms a lane each, of
+// 164,000 decisions in 9.6 and 21.6 ms.
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s) {
     if (!J.n_atoms) return;
     const uint64_t slots = (uint64_t)kEncGroups * (uint64_t)num_sms;
+    if (!J.sums) {
+        if (J.pass != RcJob::kDoubt) {
+            cudaMemsetAsync(J.doubt, 0, 4, s);
+            const uint64_t sms = (uint64_t)num_sms;
+            if (J.n_atoms <= 12 * sms) {
+                k_rc_sizes<4><<<(unsigned)((J.n_atoms + 3) / 4), 96, size_smem(4), s>>>(J);
+            } else {
+                const uint64_t nb = (J.n_atoms + 31) / 32;
+                k_rc_sizes<32><<<(unsigned)(nb < 2 * sms ? nb : 2 * sms), 768, size_smem(32), s>>>(J);
+            }
+        }
+        if (J.pass == RcJob::kNear) return;
+        const uint64_t ng = (J.n_atoms + kEncGroups - 1) / kEncGroups;
+        k_rc_encode_groups<false><<<(unsigned)(ng < (uint64_t)num_sms ? ng : (uint64_t)num_sms),
+                                    32u * kEncGroups * enc_group_warps(1), kEncGroups * enc_group_bytes(1), s>>>(J, 1);
+        return;
+    }
     if (J.n_atoms <= kGroupMax * slots) {
         const uint32_t G = (uint32_t)((J.n_atoms + slots - 1) / slots);
         const unsigned nb = (unsigned)((J.n_atoms + kEncGroups * G - 1) / (kEncGroups * G));
-        const unsigned nt = 32u * kEncGroups * enc_group_warps(G);
-        const size_t sm = kEncGroups * enc_group_bytes(G);
-        if (J.sums) k_rc_encode_groups<true><<<nb, nt, sm, s>>>(J, G);
-        else k_rc_encode_groups<false><<<nb, nt, sm, s>>>(J, G);
+        k_rc_encode_groups<true><<<nb, 32u * kEncGroups * enc_group_warps(G), kEncGroups * enc_group_bytes(G), s>>>(J,
+                                                                                                                 G);
         return;
     }
     const uint64_t k = (J.n_atoms + 32 * slots - 1) / (32 * slots);
     const uint32_t G = (uint32_t)((J.n_atoms + k * slots - 1) / (k * slots));
     const uint64_t warps = (J.n_atoms + G - 1) / G;
-    const unsigned nb = (unsigned)((warps + 3) / 4);
-    if (J.sums) k_rc_encode_lanes<true><<<nb, 128, 0, s>>>(J, G);
-    else k_rc_encode_lanes<false><<<nb, 128, 0, s>>>(J, G);
+    k_rc_encode_lanes<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(J, G);
 }
 
 void launch_consume(const PlaceJob &J, cudaStream_t s) {

@@ -60,16 +60,23 @@ struct FwdJob {
     int coef_store;
 };
 
-// Coder pass over the lists of n_atoms atoms.
+struct EncCosts;
+
+// Coder pass over the lists of n_atoms atoms: lengths, and sums or totals.
 struct RcJob {
     uint64_t n_atoms;
     const uint32_t *meta;
     const uint32_t *ent;
     uint32_t band_start[9];
     uint32_t *len;                       // payload bytes per atom ([dc] + coder bytes; 0 = zero atom)
-    uint32_t *sums;                      // optional: kSums words per atom, what k_resolve makes the bytes of
-    unsigned long long *total_bytes;     // optional: added up over the atoms
-    unsigned long long *total_present;
+    uint32_t *sums;                      // kSums words per atom, what k_resolve makes the bytes of; null: lengths alone
+    // lengths alone
+    const EncCosts *costs;
+    uint32_t *doubt;                     // scratch, 1 + n_atoms words: how many atoms only the coder can size, which
+    // both the lengths and the coder for those in doubt; the lengths alone, where
+    // an atom in doubt may be a byte longer than its length says; the coder alone
+    enum Pass { kExact, kNear, kDoubt } pass;
+    unsigned long long *totals;          // bytes, atoms present and atoms in doubt are added here
 };
 
 // Payloads from the sums of a coder pass.
@@ -99,8 +106,8 @@ struct PlaceJob {
 void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s);
 // atoms that are all LOD0 with kept coefficients: quantise and compact only
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s);
-// lengths, and the sums where J.sums is set
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s);
+void enc_costs(EncCosts *t);   // the table, on the host
 void launch_resolve(const ResolveJob &J, cudaStream_t s);
 void launch_consume(const PlaceJob &J, cudaStream_t s);
 void launch_slots(const PlaceJob &J, cudaStream_t s);

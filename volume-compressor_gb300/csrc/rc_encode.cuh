@@ -397,9 +397,9 @@ __device__ __forceinline__ void enc_zeros(EncDigits<WRITE> &e, uint32_t &q, uint
     else e.range = r;
 }
 
-template <bool WRITE, int kZ, int kU, int kB>
+template <int kZ, int kU, int kB>
 struct EncLane {
-    EncDigits<WRITE> e;
+    EncDigits<true> e;
     const uint32_t *ent;
     uint32_t *row, *ring;   // this lane's unary contexts (32 words apart) and list entries
     uint32_t nnz, i;        // list length, the entry being coded
@@ -473,7 +473,7 @@ struct EncLane {
         for (int s = 0; s < kB; ++s) {
             const bool on = have > (uint32_t)s;
             const uint32_t t = e.range >> 1;
-            if (WRITE && on && (int32_t)(bits << s) < 0) e.sum += t;
+            if (on && (int32_t)(bits << s) < 0) e.sum += t;
             e.renorm(on ? t : e.range);
         }
         const bool end = by && cnt <= (uint32_t)kB;
@@ -500,20 +500,20 @@ struct EncLane {
 
 // Every lane of the warp calls this; lanes with on code their list and return
 // the coder's byte count. mem: kEncWarpWords words of the warp.
-template <bool WRITE, int kZ, int kU, int kB>
+template <int kZ, int kU, int kB>
 __device__ __forceinline__ uint32_t enc_lanes(bool on, const uint32_t *ent, uint32_t nnz, const uint32_t *band_start,
                                               uint32_t *out, uint32_t *mem, uint32_t lane) {
-    EncLane<WRITE, kZ, kU, kB> c;
+    EncLane<kZ, kU, kB> c;
     c.init(on, ent, on ? nnz : 0u, band_start, out, mem + lane, mem + (kEncRows + 4u) * 32u + lane * kRingPitch);
     while (__any_sync(0xFFFFFFFFu, c.u != 64u)) {
         c.round(band_start);
         c.round(band_start);
-        if (WRITE && c.e.n >= kSumsMax) {
+        if (c.e.n >= kSumsMax) {
             c.over += c.e.n - (kSumsMax - 512u);
             c.e.n = kSumsMax - 512u;
         }
     }
-    if (WRITE && on) out[c.e.n] = c.e.sum;
+    if (on) out[c.e.n] = c.e.sum;
     return on ? c.e.n + c.over + 5u : 0u;
 }
 
@@ -559,6 +559,154 @@ __device__ __forceinline__ void enc_resolve(const uint32_t *sums, uint32_t n, ui
                 if (b + i < n + 5u) out[b + i] = (uint8_t)(r >> (24u - 8u * i));
         }
     }
+}
+#endif
+
+// ---------------------------------------------------------------- lengths alone
+// A decision multiplies the interval by c / 4096, c the probability of the symbol
+// it codes, up to the split's rounding down by less than one: with the interval r
+// at 2^24 or more, -log2 of the factor lies within 4096 log2(e) / (2^24 c) of
+// 12 - log2 c, above it below the split and below it above. So the bits L by
+// which a list's decisions shrink the interval are known, to about a hundredth
+// of a bit, from their probabilities alone, without the interval: in any order,
+// a lane per context. And the renormalisations leave the interval in
+// [2^24, 2^32), so their number is L / 8 rounded down unless L is that close to a
+// multiple of 8 (one atom in a thousand), where the coder has to run.
+//
+// Costs are in 2^-26 bits, rounded to the nearest; a table entry is a cost and
+// the most that the true one can differ from it.
+constexpr uint32_t kCostOne = 1u << 26;    // one bit
+constexpr uint32_t kCostSlack = 1u;        // of the rounding, either way
+constexpr uint32_t kCostBypass = 6u;       // a bypass decision: one bit and at most 1.45 2^-24 more
+struct EncCosts {
+    uint2 one[4096];     // [c]: cost, error
+    uint2 eight[4096];   // [q]: eight zeros from q = 4096 - p: cost, error << 16 | q after them
+};
+
+#ifdef __CUDACC__
+struct EncSize {   // least and most bits are cost - lo and cost + hi
+    uint64_t cost;
+    uint32_t lo, hi;
+};
+
+// Significance decisions of band b of the lane's atom: up to eight and four zeros
+// and the nonzero a round, as enc_lanes. ROW: lanes 8i..8i+7 hold an atom's bands.
+template <bool ROW>
+__device__ __forceinline__ EncSize enc_size_bands(const EncCosts &T, const uint32_t *ent, uint32_t nnz, uint32_t b,
+                                                  const uint32_t *band_start, uint32_t *ring) {
+    EncSize r{0, 0, 0};
+    const uint32_t eob = nnz ? (ent[nnz - 1u] & 0xFFFFu) + 1u : 0u;
+    const uint32_t beg = band_start[b];
+    auto first = [&](uint32_t at) {   // the first entry from scan position at on
+        uint32_t lo = 0;
+        for (uint32_t hi = nnz; lo < hi;) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if ((ent[mid] & 0xFFFFu) < at) lo = mid + 1u;
+            else hi = mid;
+        }
+        return lo;
+    };
+    uint32_t e = first(beg);
+    uint32_t e1;
+    if (ROW) {
+        e1 = __shfl_down_sync(0xFFFFFFFFu, e, 1);
+        e1 = b == 7u ? nnz : e1;
+    } else {
+        e1 = first(band_start[b + 1u]);
+    }
+    const uint32_t end = band_start[b + 1u] < eob ? band_start[b + 1u] : eob;
+    bool live = beg < end;
+    const uint32_t j0 = e & ~3u;
+#pragma unroll
+    for (uint32_t k = 0; k < kRingAhead; ++k)
+        if (live && j0 + 4u * k < e1) ring_copy(ring + (j0 + 4u * k) % kRing, ent + j0 + 4u * k);
+    ring_commit();
+    ring_wait<0>();
+    uint32_t p = live && e < e1 ? ring[e % kRing] & 0xFFFFu : end;
+    uint32_t rem = live ? p - beg : 0u, q = 2048u;
+    if (live) {   // the slack of every zero, or eight of them, and of every nonzero
+        r.lo = (end - beg) * kCostSlack;
+        r.hi = (e1 - e) * kCostSlack;
+    }
+    auto round = [&]() {
+        const uint32_t nx = ring[(e + 1u) % kRing] & 0xFFFFu;
+        uint32_t sum = 0;   // at most 64 bits: eight zeros cost 30 at most, four 20
+        {
+            const uint2 v = T.eight[q];
+            const bool on = rem >= 8u;
+            sum += on ? v.x : 0u;
+            r.hi += on ? v.y >> 16 : 0u;
+            q = on ? v.y & 0xFFFFu : q;
+            rem -= on ? 8u : 0u;
+        }
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const uint2 v = T.one[4096u - q];
+            const bool on = rem > (uint32_t)y;
+            sum += on ? v.x : 0u;
+            r.hi += on ? v.y : 0u;
+            q = on ? q - (q >> 5) : q;
+        }
+        rem -= rem < 4u ? rem : 4u;
+        const bool ev = live && rem == 0u, hit = ev && e < e1;
+        const uint2 v = T.one[q];
+        sum += hit ? v.x : 0u;
+        r.lo += hit ? v.y : 0u;
+        q += hit ? (4096u - q) >> 5 : 0u;
+        e += hit ? 1u : 0u;
+        const uint32_t np = e < e1 ? nx : end;
+        rem = hit ? np - p - 1u : rem;
+        p = hit ? np : p;
+        live = live && (!ev || hit);
+        const uint32_t j = (e & ~3u) + 4u * (kRingAhead - 1u);
+        if (hit && (e & 3u) == 0u && j < e1) ring_copy(ring + j % kRing, ent + j);
+        r.cost += sum;
+    };
+    while (__any_sync(0xFFFFFFFFu, live)) {
+        round();
+        round();
+        ring_commit();
+        ring_wait<4>();
+    }
+    ring_wait<0>();   // the ring is the next atom's
+    return r;
+}
+
+// The other decisions: lane k of each sixteen steps unary context k through its
+// atom's list, lane j counts the bypass decisions of every sixteenth entry.
+__device__ __forceinline__ EncSize enc_size_rest(const EncCosts &T, const uint32_t *ent, uint32_t nnz,
+                                                 uint32_t lane) {
+    EncSize r{0, 0, 0};
+    const uint32_t l = lane & 15u;
+    const uint32_t clane = l < 12u ? l : 0xFFFFu, clane1 = clane + 1u;
+    const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, nnz);
+    uint32_t ctx = 2048u, nx = l < nnz ? __ldg(ent + l) : 0u;
+    for (uint32_t i0 = 0; i0 < most; i0 += 16u) {
+        const int32_t lv = (int32_t)nx >> 16;
+        const uint32_t m = (uint32_t)(lv < 0 ? -lv : lv);   // 0 past the list's end
+        nx = i0 + 16u + l < nnz ? __ldg(ent + i0 + 16u + l) : 0u;
+        uint32_t bits;
+        const uint32_t tail = m ? enc_tail(m, false, &bits) : 0u;
+        r.cost += (uint64_t)tail * kCostOne;
+        r.hi += tail * kCostBypass;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t sum = 0;   // eight decisions of at most 7.05 bits
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t mj = __shfl_sync(0xFFFFFFFFu, m, h * 8 + j, 16);
+                const bool has = mj > clane, b = mj > clane1;
+                const uint2 v = T.one[b ? 4096u - ctx : ctx];
+                sum += has ? v.x : 0u;
+                r.lo += has ? (b ? v.y : kCostSlack) : 0u;
+                r.hi += has ? (b ? kCostSlack : v.y) : 0u;
+                const uint32_t nc = ctx + (uint32_t)((int32_t)((b ? 31u : 4096u) - ctx) >> 5);
+                ctx = has ? nc : ctx;
+            }
+            r.cost += sum;
+        }
+    }
+    return r;
 }
 #endif
 

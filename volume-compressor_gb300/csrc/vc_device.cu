@@ -6,7 +6,9 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "k_encode.cuh"
 #include "kernels.cuh"
+#include "rc_encode.cuh"
 #include "vc_device.h"
 
 using namespace vcg;
@@ -50,6 +52,16 @@ static void init_once(void) {
         return;
     }
     free(t);
+    EncCosts *ec = (EncCosts *)malloc(sizeof(EncCosts));
+    if (!ec) { snprintf(g_err, sizeof g_err, "cost table: out of memory"); return; }
+    enc_costs(ec);
+    if ((e = cudaMalloc(&g_dev.costs, sizeof(EncCosts))) != cudaSuccess ||
+        (e = cudaMemcpy(g_dev.costs, ec, sizeof(EncCosts), cudaMemcpyHostToDevice)) != cudaSuccess) {
+        vcd_set_error("cost table upload", e);
+        free(ec);
+        return;
+    }
+    free(ec);
     __atomic_store_n(&g_init_rc, 0, __ATOMIC_RELEASE);
 }
 

@@ -35,13 +35,15 @@ struct EncState {
     Layout lay;
     const uint8_t *lvol[8];
     uint32_t dims[8][3];
-    uint32_t *ent, *meta, *len, *best;   // lists and meta: LOD0's, or a chunk's
+    uint32_t *ent, *meta, *len;          // lists and meta: LOD0's, or a chunk's
     uint32_t *ent2, *meta2;              // the coarser LODs', beside them (null: none)
+    uint32_t *doubt, *doubt2;            // a size pass's scratch beside meta and meta2
     uint32_t *sums;                      // the coder's sums, kSums words an atom
     bool whole;                          // lists and sums of every atom are kept: one coder pass
     uint64_t *pos;
     uint8_t *dc, *arc;
-    unsigned long long *red;
+    unsigned long long *red;             // a size pass's totals: bytes, atoms present, atoms in doubt
+    RcJob::Pass size_pass;
     vcd_quant *qtab;          // device, per LOD
     vcd_quant qh;             // host staging
     // LOD0 forward transform kept across passes, packed (null when it does not fit)
@@ -136,8 +138,10 @@ static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaS
     memcpy(R.band_start, g_dev.band_start, sizeof R.band_start);
     R.len = S.len + c0;
     if (pass == kSizes) {
-        R.total_bytes = S.red;
-        R.total_present = S.red + 1;
+        R.costs = (const EncCosts *)g_dev.costs;
+        R.doubt = meta == S.meta ? S.doubt : S.doubt2;
+        R.pass = S.size_pass;
+        R.totals = S.red;
     } else {
         // without room for sums the payloads are coded from the lists (kWrite)
         R.sums = pass == kCode ? sums + c0 * kSums : sums;
@@ -257,15 +261,15 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     CK(vcd_scratch(c, VCD_BUF_EENT, chunk * VCD_MAX_ENTRIES * 4 + 16, &p), "coefficient lists");
     S.ent = (uint32_t *)p;
     const uint64_t na0 = S.lay.base[1];
-    // quant table (8 LODs) | meta (chunk) | len (all atoms) | best LOD0 len | dc (all atoms)
-    size_t q_b = 8 * sizeof(vcd_quant), meta_b = chunk * 4, len_b = total_atoms * 4, best_b = na0 * 4;
+    // quant table (8 LODs) | meta (chunk) | doubt (1 + chunk) | len (all atoms) | dc (all atoms)
+    size_t q_b = 8 * sizeof(vcd_quant), meta_b = chunk * 4, doubt_b = (chunk + 1) * 4, len_b = total_atoms * 4;
     size_t dc_b = total_atoms + 16;
-    CK(vcd_scratch(c, VCD_BUF_EMETA, q_b + meta_b + len_b + best_b + dc_b + 64, &p), "encode metadata");
+    CK(vcd_scratch(c, VCD_BUF_EMETA, q_b + meta_b + doubt_b + len_b + dc_b + 64, &p), "encode metadata");
     S.qtab = (vcd_quant *)p;
     S.meta = (uint32_t *)((uint8_t *)p + q_b);
-    S.len = S.meta + chunk;
-    S.best = S.len + total_atoms;
-    S.dc = (uint8_t *)(S.best + na0);
+    S.doubt = S.meta + chunk;
+    S.len = S.doubt + chunk + 1;
+    S.dc = (uint8_t *)(S.len + total_atoms);
     CK(vcd_scratch(c, VCD_BUF_POS, (total_atoms + 1) * 8, &p), "placement");
     S.pos = (uint64_t *)p;
     CK(vcd_scratch(c, VCD_BUF_RED, 64, &p), "totals");
@@ -288,9 +292,10 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         const size_t all_b = (size_t)total_atoms * kSums * 4;
         void *pe = NULL, *pm = NULL;
         if (n1 && vcd_scratch(c, VCD_BUF_EENT2, n1c * VCD_MAX_ENTRIES * 4 + 16, &pe) == cudaSuccess &&
-            vcd_scratch(c, VCD_BUF_EMETA2, n1c * 4 + 16, &pm) == cudaSuccess) {
+            vcd_scratch(c, VCD_BUF_EMETA2, n1c * 8 + 16, &pm) == cudaSuccess) {
             S.ent2 = (uint32_t *)pe;
             S.meta2 = (uint32_t *)pm;
+            S.doubt2 = S.meta2 + n1c;
         }
         if (na0 <= kChunk && n1 <= kChunk && (S.ent2 || !n1) && cudaMemGetInfo(&fr, &tot) == cudaSuccess &&
             (c->cap[VCD_BUF_ESUM] >= all_b || all_b <= fr / 2) &&
@@ -303,34 +308,77 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         cudaGetLastError();
     }
 
-    // ---- rate control on LOD0 (bisection over float bit patterns of [0.05, 4096])
+    // ---- rate control on LOD0 (bisection over float bit patterns of [0.05, 4096]):
+    // the q visited whose ratio is nearest the target, the larger of two as near.
+    // A pass that leaves d atoms in doubt knows its bytes up to d. Those atoms are
+    // coded where that decides the next step or is likely to decide the best, or
+    // after the last step for a q that may still be the nearest.
+    struct Visit { float q; unsigned long long bytes, present, doubt; } v[24];
+    const double target = (double)info->target_ratio;
+    auto measure = [&](Visit &m, RcJob::Pass pass) -> cudaError_t {
+        cudaError_t e = cudaSuccess;
+        S.size_pass = pass;
+        if (pass == RcJob::kDoubt) {   // the lists are those of the pass before
+            code_chunk(S, 0, na0, kSizes, st, S.ent, S.meta, nullptr);
+        } else {
+            if ((e = cudaMemsetAsync(S.red, 0, 24, st)) != cudaSuccess) return e;
+            set_q(S, 0, m.q);
+            run_range(S, 0, na0, kSizes, st, S.ent, S.meta);
+        }
+        unsigned long long h[3];
+        if ((e = cudaMemcpyAsync(h, S.red, 24, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+        m.bytes = h[0];
+        m.present = h[1];
+        m.doubt = pass == RcJob::kNear ? h[2] : 0;
+        return cudaSuccess;
+    };
+    auto ratio = [](const Visit &m, unsigned long long more) {
+        return (double)(32768ull * m.present) / (double)(m.bytes + more);
+    };
     uint32_t lo = b_of(0.05f), hi = b_of(4096.0f);
     float best_q = 1.0f;
     double best_err = INFINITY;
     uint64_t present = 0, best_bytes = 0;
-    bool have_best = false;
+    int nv = 0;
     for (int it = 0; it < (info->fixed_q ? 0 : 24); ++it) {
         uint32_t mid = lo + (hi - lo) / 2;
-        float q = f_of(mid);
-        CK(cudaMemsetAsync(S.red, 0, 16, st), "totals reset");
-        set_q(S, 0, q);
-        run_range(S, 0, na0, kSizes, st, S.ent, S.meta);
-        unsigned long long h[2];
-        CK(cudaMemcpyAsync(h, S.red, 16, cudaMemcpyDeviceToHost, st), "totals read");
-        CK(cudaStreamSynchronize(st), "rate control pass");
-        present = h[1];
+        Visit &m = v[nv];
+        m.q = f_of(mid);
+        CK(measure(m, RcJob::kNear), "rate control pass");
+        present = m.present;
         if (present == 0) break;
-        double ratio = (double)(32768ull * present) / (double)h[0];
-        double err = fabs(ratio - (double)info->target_ratio);
-        if (err < best_err || (err == best_err && q > best_q)) {
-            best_err = err;
-            best_q = q;
-            best_bytes = h[0];
-            have_best = true;
-            if (!S.whole) CK(cudaMemcpyAsync(S.best, S.len, na0 * 4, cudaMemcpyDeviceToDevice, st), "keep sizes");
-        }
-        if (ratio < (double)info->target_ratio) lo = mid; else hi = mid;
+        // the doubt of a pass this near is likely to matter, and its lists are at hand
+        const double want = (double)(32768ull * m.present) / target;
+        if ((ratio(m, m.doubt) < target) != (ratio(m, 0) < target) ||
+            fabs((double)m.bytes - want) <= 4.0 * (double)m.doubt)
+            if (m.doubt) CK(measure(m, na0 <= kChunk ? RcJob::kDoubt : RcJob::kExact), "rate control pass");
+        if (ratio(m, 0) < target) lo = mid; else hi = mid;
+        ++nv;
     }
+    auto consider = [&](const Visit &m) {
+        const double err = fabs(ratio(m, 0) - target);
+        if (err < best_err || (err == best_err && m.q > best_q)) {
+            best_err = err;
+            best_q = m.q;
+            best_bytes = m.bytes;
+        }
+    };
+    for (int i = 0; i < nv; ++i)
+        if (!v[i].doubt) consider(v[i]);
+    for (;;) {   // the nearest that one in doubt can be, until none can be nearer than the best
+        int near = -1;
+        double near_err = best_err;
+        for (int i = 0; i < nv; ++i) {
+            const double e = v[i].doubt ? fmin(fabs(ratio(v[i], 0) - target), fabs(ratio(v[i], v[i].doubt) - target))
+                                        : INFINITY;
+            if (v[i].doubt && e <= near_err) near = i, near_err = e;
+        }
+        if (near < 0) break;
+        CK(measure(v[near], RcJob::kExact), "rate control pass");
+        consider(v[near]);
+    }
+    S.size_pass = RcJob::kExact;
     info->q0 = best_q;
     info->present0 = present;
     info->bytes0 = best_bytes;
@@ -347,11 +395,8 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     for (int l = 0; l < nlod; ++l) set_q(S, l, qs[l]);
     if (S.whole) {
         run_split(S, na0, total_atoms, chunk, kCode);
-    } else if (have_best) {
-        CK(cudaMemcpyAsync(S.len, S.best, na0 * 4, cudaMemcpyDeviceToDevice, st), "restore sizes");
-        run_range(S, na0, total_atoms, kSizes, st, S.ent, S.meta);
     } else {
-        CK(cudaMemsetAsync(S.red, 0, 16, st), "totals reset");
+        CK(cudaMemsetAsync(S.red, 0, 24, st), "totals reset");
         run_split(S, na0, total_atoms, chunk, kSizes);
     }
 
