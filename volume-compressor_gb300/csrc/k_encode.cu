@@ -24,7 +24,11 @@
 
 namespace vcg {
 
-constexpr int kFwdThreads = 256;
+// k_fwd holds an atom's tile and levels, so an SM runs one CTA: 16 warps of it,
+// two rows or lines a thread, hide each other's latency (the 37,451 atoms of a
+// 1024^3 pyramid in 6.9 ms; 8 warps and the transform kept for later passes, 8.7).
+constexpr int kFwdThreads = 512;
+constexpr int kQuantThreads = 256;
 constexpr size_t kFwdSmem = kTileBytes + 32768 * sizeof(int16_t);
 
 // 32 voxels of row (z, y) of atom (az, ay, ax), zero outside the volume, packed
@@ -77,23 +81,24 @@ __device__ __forceinline__ int32_t quant_packed(uint32_t w, const float *qdz, co
 
 // Quantise one atom in scan order and compact its nonzero levels into the list
 // dst (scan position | level << 16, in scan order); returns the count (every
-// thread). Warp w owns scan positions [4096 w, 4096 w + 4096), 128 at a time,
+// thread). Warp w owns kPer scan positions from kPer w on, 128 at a time,
 // each lane 4 consecutive ones (pk4(p) gives the packed coefficients of scan
 // positions p..p+3): pass 1 quantises, keeps the levels in lv and counts them;
 // pass 2 places each lane's entries after a warp prefix sum of the per-lane
-// counts, skipping groups without a nonzero level. NT must be 256.
+// counts, skipping groups without a nonzero level.
 template <int NT, class Pk4>
 __device__ __forceinline__ uint32_t quant_compact(Pk4 &&pk4, const float *qdz, const float *qrr, int16_t *lv,
                                                   uint32_t *wcnt, uint32_t *dst) {
-    static_assert(NT == 256, "eight warps of 4096 scan positions");
+    constexpr uint32_t kPer = 32768 / (NT / 32);
+    static_assert(kPer % 512 == 0, "whole groups of loads");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t p0 = (uint32_t)warp * 4096u + 4u * (uint32_t)lane;
+    const uint32_t p0 = (uint32_t)warp * kPer + 4u * (uint32_t)lane;
     uint32_t cnt = 0;
     // groups of kG x 128 positions: every load of a group is issued before the
     // first level is stored
     constexpr uint32_t kG = 4;
 #pragma unroll 1
-    for (uint32_t i = 0; i < 4096; i += 128 * kG) {
+    for (uint32_t i = 0; i < kPer; i += 128 * kG) {
         uint4 w[kG];
 #pragma unroll
         for (uint32_t g = 0; g < kG; ++g) w[g] = pk4(p0 + i + 128 * g);
@@ -117,7 +122,7 @@ __device__ __forceinline__ uint32_t quant_compact(Pk4 &&pk4, const float *qdz, c
         total += v;
     }
 #pragma unroll 4
-    for (uint32_t i = 0; i < 4096; i += 128) {
+    for (uint32_t i = 0; i < kPer; i += 128) {
         const uint32_t p = p0 + i;
         const uint2 pk = *reinterpret_cast<const uint2 *>(lv + p);
         if (!__any_sync(0xFFFFFFFFu, (pk.x | pk.y) != 0u)) continue;
@@ -182,11 +187,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
         } else {
             const uint8_t *vol = J.vol[lod];
             const uint32_t nx = J.dims[lod][0], ny = J.dims[lod][1], nz = J.dims[lod][2];
-            // rows r = tid + 256 j: z = r >> 5, y = r & 31 (lane)
-            uint32_t w[4][8];
+            // rows r = tid + kFwdThreads j: z = r >> 5, y = r & 31 (lane)
+            constexpr int kRows = 1024 / kFwdThreads;
+            uint32_t w[kRows][8];
             uint32_t s = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < kRows; ++j) {
                 int r = tid + kFwdThreads * j;
                 load_row(vol, nx, ny, nz, ax * 32, ay * 32 + (r & 31), az * 32 + (r >> 5), w[j]);
 #pragma unroll
@@ -209,9 +215,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
             }
             dc = (int32_t)((sum + 16384u) / 32768u);
             if (cached && tid == 0) J.coef_dc[ca] = (uint32_t)dc;
-            // pass along x for the thread's 4 rows, straight from registers
+            // pass along x for the thread's rows, straight from registers
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < kRows; ++j) {
                 int r = tid + kFwdThreads * j;
                 int32_t v[32], o[32];
 #pragma unroll
@@ -262,12 +268,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
 // a quarter of the shared memory of k_fwd (three CTAs per SM).
 constexpr size_t kQuantSmem = 32768 * sizeof(int16_t);
 
-__global__ void __launch_bounds__(kFwdThreads) k_quant_cached(FwdJob J) {
+__global__ void __launch_bounds__(kQuantThreads) k_quant_cached(FwdJob J) {
     extern __shared__ int16_t lv[];
     __shared__ float qdz[VCD_NCLASS], qrr[VCD_NCLASS];
-    __shared__ uint32_t wcnt[kFwdThreads / 32];
+    __shared__ uint32_t wcnt[kQuantThreads / 32];
     const int tid = threadIdx.x;
-    for (int i = tid; i < VCD_NCLASS; i += kFwdThreads) { qdz[i] = J.q[0].dz[i]; qrr[i] = J.q[0].rr[i]; }
+    for (int i = tid; i < VCD_NCLASS; i += kQuantThreads) { qdz[i] = J.q[0].dz[i]; qrr[i] = J.q[0].rr[i]; }
     __syncthreads();
     for (uint64_t t = blockIdx.x; t < J.n_atoms; t += gridDim.x) {
         const uint64_t ca = J.first + t;
@@ -277,7 +283,7 @@ __global__ void __launch_bounds__(kFwdThreads) k_quant_cached(FwdJob J) {
             continue;
         }
         const uint32_t *cptr = J.coef + ca * 32768ull;
-        const uint32_t total = quant_compact<kFwdThreads>(
+        const uint32_t total = quant_compact<kQuantThreads>(
             [&](uint32_t p) { return __ldcs(reinterpret_cast<const uint4 *>(cptr + p)); }, qdz, qrr, lv, wcnt,
             J.ent + t * (uint64_t)VCD_MAX_ENTRIES);
         if (tid == 0) J.meta[t] = total | ((dcz & 0xFFu) << 16);
@@ -391,13 +397,15 @@ __global__ void __launch_bounds__(24 * A) k_rc_sizes(RcJob J) {
 }
 
 // Many atoms: a lane each, G per warp.
-__global__ void __launch_bounds__(128) k_rc_encode_lanes(RcJob J, uint32_t G) {
+constexpr uint32_t kLanesWarps = 4;
+
+__global__ void __launch_bounds__(32 * kLanesWarps) k_rc_encode_lanes(RcJob J, uint32_t G) {
     __shared__ uint32_t bstart[9];
-    __shared__ __align__(16) uint32_t mem[4][kEncWarpWords];
+    __shared__ __align__(16) uint32_t mem[kLanesWarps][kEncWarpWords];
     if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t t = lane < G ? ((uint64_t)blockIdx.x * 4u + warp) * G + lane : J.n_atoms;
+    const uint64_t t = lane < G ? ((uint64_t)blockIdx.x * kLanesWarps + warp) * G + lane : J.n_atoms;
     const uint32_t *ent;
     uint32_t nnz;
     const bool on = enc_atom(J, t, ent, nnz);
@@ -479,7 +487,7 @@ void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s) {
     enc_set_smem();
     if (!J.n_atoms) return;
     const uint64_t cap = (uint64_t)num_sms * 3;
-    k_quant_cached<<<(unsigned)(J.n_atoms < cap ? J.n_atoms : cap), kFwdThreads, kQuantSmem, s>>>(J);
+    k_quant_cached<<<(unsigned)(J.n_atoms < cap ? J.n_atoms : cap), kQuantThreads, kQuantSmem, s>>>(J);
 }
 
 void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s) {
@@ -517,6 +525,8 @@ void enc_costs(EncCosts *t) {
 // sub-partition that hold them at 32 a warp, spread evenly. At the line: 4,681
 // atoms of 30,000 decisions in 2.6 ms as groups of 8 and 3.2 ms a lane each, of
 // 164,000 decisions in 9.6 and 21.6 ms.
+uint64_t enc_group_atoms(int num_sms) { return (uint64_t)kGroupMax * kEncGroups * (uint64_t)num_sms; }
+
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s) {
     if (!J.n_atoms) return;
     const uint64_t slots = (uint64_t)kEncGroups * (uint64_t)num_sms;
@@ -537,17 +547,17 @@ void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s) {
                                     32u * kEncGroups * enc_group_warps(1), kEncGroups * enc_group_bytes(1), s>>>(J, 1);
         return;
     }
-    if (J.n_atoms <= kGroupMax * slots) {
+    if (J.n_atoms <= enc_group_atoms(num_sms)) {
         const uint32_t G = (uint32_t)((J.n_atoms + slots - 1) / slots);
         const unsigned nb = (unsigned)((J.n_atoms + kEncGroups * G - 1) / (kEncGroups * G));
-        k_rc_encode_groups<true><<<nb, 32u * kEncGroups * enc_group_warps(G), kEncGroups * enc_group_bytes(G), s>>>(J,
-                                                                                                                 G);
+        const unsigned nt = 32u * kEncGroups * enc_group_warps(G);
+        k_rc_encode_groups<true><<<nb, nt, kEncGroups * enc_group_bytes(G), s>>>(J, G);
         return;
     }
     const uint64_t k = (J.n_atoms + 32 * slots - 1) / (32 * slots);
     const uint32_t G = (uint32_t)((J.n_atoms + k * slots - 1) / (k * slots));
     const uint64_t warps = (J.n_atoms + G - 1) / G;
-    k_rc_encode_lanes<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(J, G);
+    k_rc_encode_lanes<<<(unsigned)((warps + kLanesWarps - 1) / kLanesWarps), 32 * kLanesWarps, 0, s>>>(J, G);
 }
 
 void launch_consume(const PlaceJob &J, cudaStream_t s) {

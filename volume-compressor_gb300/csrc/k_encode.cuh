@@ -108,6 +108,8 @@ void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s);
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s);
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s);
 void enc_costs(EncCosts *t);   // the table, on the host
+// atoms that a coder pass runs as groups at most
+uint64_t enc_group_atoms(int num_sms);
 void launch_resolve(const ResolveJob &J, cudaStream_t s);
 void launch_consume(const PlaceJob &J, cudaStream_t s);
 void launch_slots(const PlaceJob &J, cudaStream_t s);

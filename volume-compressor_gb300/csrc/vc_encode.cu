@@ -172,7 +172,10 @@ static void run_range(EncState &S, uint64_t a0, uint64_t a1, EncPass pass, cudaS
 // beside it on the second stream, with their own list scratch. The coarser LODs
 // are few atoms but the finest-quantised ones (q down to 0.05): one of them is a
 // serial coder chain longer than a whole LOD0 pass, so run after LOD0 it would
-// add its length. Serial under per-stage measurement (its events are per stream).
+// add its length. Where each range is one chunk and LOD0 more than the coder's
+// groups hold, both coders fill the GPU and only get in each other's way (one
+// after the other 13.9 ms at 1024^3, side by side 12 to 25). Serial under
+// per-stage measurement (its events are per stream).
 static void run_split(EncState &S, uint64_t na0, uint64_t total, uint64_t chunk, EncPass pass) {
     vcd_ctx *c = S.c;
     // chunks of a kWrite have their own sums on each stream
@@ -181,11 +184,12 @@ static void run_split(EncState &S, uint64_t na0, uint64_t total, uint64_t chunk,
         run_range(S, 0, total, pass, c->stream, S.ent, S.meta, S.sums);
         return;
     }
-    cudaStream_t side = vcd_prof_on() ? NULL : vcd_side_stream(c), st1 = side ? side : c->stream;
+    const bool first = total - na0 <= kChunk && na0 <= kChunk;
+    const bool alone = first && na0 > enc_group_atoms(g_dev.num_sms);
+    cudaStream_t side = alone || vcd_prof_on() ? NULL : vcd_side_stream(c), st1 = side ? side : c->stream;
     // A forward CTA takes nearly all shared memory of an SM, so beside a coder it
     // waits for the coder's CTAs: where one chunk holds each range, both forward
     // passes go first and only the coders run side by side.
-    const bool first = total - na0 <= kChunk && na0 <= kChunk;
     if (first) {
         fwd_chunk(S, na0, total - na0, c->stream, S.ent2, S.meta2);
         fwd_chunk(S, 0, na0, c->stream, S.ent, S.meta);
@@ -274,7 +278,9 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     S.pos = (uint64_t *)p;
     CK(vcd_scratch(c, VCD_BUF_RED, 64, &p), "totals");
     S.red = (unsigned long long *)p;
-    {   // keep LOD0's forward transform (128 KiB per atom) when it takes at most half the free memory
+    // keep LOD0's forward transform (128 KiB per atom) for the passes after the first when it takes at most half the
+    // free memory
+    auto keep_coef = [&]() {
         size_t fr = 0, tot = 0;
         const size_t cb = (size_t)na0 * 131072 + (size_t)na0 * 4 + 64;
         if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && (c->cap[VCD_BUF_COEF] >= cb || cb <= fr / 2) &&
@@ -284,7 +290,8 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
             S.coef_n = na0;
         }
         cudaGetLastError();
-    }
+    };
+    if (!info->fixed_q) keep_coef();
     {   // One coder pass for all where the lists and sums of every atom have room (256 KiB an atom, the sums
         // in at most half the free memory): else one for the sizes and one, a chunk at a time, for the bytes.
         size_t fr = 0, tot = 0;
@@ -307,6 +314,7 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         }
         cudaGetLastError();
     }
+    if (info->fixed_q && !S.whole) keep_coef();   // one pass keeps nothing
 
     // ---- rate control on LOD0 (bisection over float bit patterns of [0.05, 4096]):
     // the q visited whose ratio is nearest the target, the larger of two as near.
