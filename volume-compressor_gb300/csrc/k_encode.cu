@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(32 * kEncGroups * enc_group_warps(kGroupMax)) 
             const uint32_t eob = nnz ? (ent[nnz - 1u] & 0xFFFFu) + 1u : 0u;
             const uint32_t k = enc_consume<SUMS>(g, on, eob, SUMS ? J.sums + (on ? t : 0) * kSums : nullptr, lane);
             if (t < J.n_atoms) {
-                if (!SUMS && on) atomicAdd(J.totals, (unsigned long long)(k + 1u - J.len[t]));
+                if (!SUMS && on) atomicAdd(J.totals + 3 * (t / J.per), (unsigned long long)(k + 1u - J.len[t]));
                 J.len[t] = on ? k + 1u : 0u;
             }
         } else {
@@ -384,6 +384,15 @@ __global__ void __launch_bounds__(24 * A) k_rc_sizes(RcJob J) {
             if (!(m & 0xFFFFu)) n = 2u, sure = true;   // 16 halvings of 2^32 - 1
             if (t < J.n_atoms) J.len[t] = on ? n + 6u : 0u;
             if (on && !sure) J.doubt[1u + atomicAdd(J.doubt, 1u)] = (uint32_t)t;
+            if (A == 4) {   // its atoms may be of two sets
+                if (on) {
+                    unsigned long long *tot = J.totals + 3 * (t / J.per);
+                    atomicAdd(tot, n + 6ull);
+                    atomicAdd(tot + 1, 1ull);
+                    if (!sure) atomicAdd(tot + 2, 1ull);
+                }
+                continue;
+            }
             const uint32_t bytes = __reduce_add_sync(0xFFFFFFFFu, on ? n + 6u : 0u);
             const uint32_t present = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, on));
             const uint32_t doubt = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, on && !sure));
@@ -525,6 +534,8 @@ void enc_costs(EncCosts *t) {
 // sub-partition that hold them at 32 a warp, spread evenly. At the line: 4,681
 // atoms of 30,000 decisions in 2.6 ms as groups of 8 and 3.2 ms a lane each, of
 // 164,000 decisions in 9.6 and 21.6 ms.
+uint64_t size_sets_atoms(int num_sms) { return 12ull * (uint64_t)num_sms; }
+
 uint64_t enc_group_atoms(int num_sms) { return (uint64_t)kGroupMax * kEncGroups * (uint64_t)num_sms; }
 
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s) {
@@ -534,7 +545,7 @@ void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s) {
         if (J.pass != RcJob::kDoubt) {
             cudaMemsetAsync(J.doubt, 0, 4, s);
             const uint64_t sms = (uint64_t)num_sms;
-            if (J.n_atoms <= 12 * sms) {
+            if (J.n_atoms <= size_sets_atoms(num_sms)) {
                 k_rc_sizes<4><<<(unsigned)((J.n_atoms + 3) / 4), 96, size_smem(4), s>>>(J);
             } else {
                 const uint64_t nb = (J.n_atoms + 31) / 32;

@@ -76,7 +76,8 @@ struct RcJob {
     // both the lengths and the coder for those in doubt; the lengths alone, where
     // an atom in doubt may be a byte longer than its length says; the coder alone
     enum Pass { kExact, kNear, kDoubt } pass;
-    unsigned long long *totals;          // bytes, atoms present and atoms in doubt are added here
+    unsigned long long *totals;          // bytes, atoms present and atoms in doubt are added here, for every set
+    uint64_t per;                        // of `per` atoms its own three (sets of more than size_sets_atoms: one set)
 };
 
 // Payloads from the sums of a coder pass.
@@ -108,6 +109,8 @@ void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s);
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s);
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s);
 void enc_costs(EncCosts *t);   // the table, on the host
+// atoms that a pass for lengths takes as sets, or at once four a CTA, at most
+uint64_t size_sets_atoms(int num_sms);
 // atoms that a coder pass runs as groups at most
 uint64_t enc_group_atoms(int num_sms);
 void launch_resolve(const ResolveJob &J, cudaStream_t s);

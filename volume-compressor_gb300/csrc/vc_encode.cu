@@ -44,6 +44,7 @@ struct EncState {
     uint8_t *dc, *arc;
     unsigned long long *red;             // a size pass's totals: bytes, atoms present, atoms in doubt
     RcJob::Pass size_pass;
+    uint32_t sets;                       // quantisers a size pass takes at once, LOD0's lists of each after the other
     vcd_quant *qtab;          // device, per LOD
     vcd_quant qh;             // host staging
     // LOD0 forward transform kept across passes, packed (null when it does not fit)
@@ -93,7 +94,8 @@ static void resolve_range(EncState &S, uint64_t c0, uint64_t n, const uint32_t *
 }
 
 // forward pass over canonical atoms [c0, c0 + n)
-static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uint32_t *ent, uint32_t *meta) {
+static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uint32_t *ent, uint32_t *meta,
+                      uint32_t set = 0) {
     FwdJob F;
     memset(&F, 0, sizeof F);   // fields this pass does not use stay null
     F.lay = S.lay;
@@ -101,7 +103,7 @@ static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uin
     memcpy(F.dims, S.dims, sizeof F.dims);
     F.first = c0;
     F.n_atoms = n;
-    F.q = S.qtab;
+    F.q = S.qtab + set;
     F.scan = g_dev.tables->scan;
     F.alt_mask = g_dev.tables->alt_mask;
     F.ent = ent;
@@ -138,6 +140,8 @@ static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaS
     memcpy(R.band_start, g_dev.band_start, sizeof R.band_start);
     R.len = S.len + c0;
     if (pass == kSizes) {
+        R.n_atoms = n * S.sets;
+        R.per = n;
         R.costs = (const EncCosts *)g_dev.costs;
         R.doubt = meta == S.meta ? S.doubt : S.doubt2;
         R.pass = S.size_pass;
@@ -261,22 +265,27 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         vcd_prof_add("downsample", vcd_elapsed(c->ev[6], c->ev[5]), (uint64_t)(nlod - 1), nvox[0] + pyr_vox - nvox[nlod - 1],
                      pyr_vox, pyr_vox);
     }
-    const uint64_t chunk = total_atoms < kChunk ? total_atoms : kChunk;
-    CK(vcd_scratch(c, VCD_BUF_EENT, chunk * VCD_MAX_ENTRIES * 4 + 16, &p), "coefficient lists");
-    S.ent = (uint32_t *)p;
     const uint64_t na0 = S.lay.base[1];
-    // quant table (8 LODs) | meta (chunk) | doubt (1 + chunk) | len (all atoms) | dc (all atoms)
-    size_t q_b = 8 * sizeof(vcd_quant), meta_b = chunk * 4, doubt_b = (chunk + 1) * 4, len_b = total_atoms * 4;
+    const uint64_t chunk = total_atoms < kChunk ? total_atoms : kChunk;
+    // a rate control of few atoms takes three quantisers at once
+    const bool three = !info->fixed_q && 3 * na0 <= size_sets_atoms(g_dev.num_sms);
+    const uint64_t lists = three && 3 * na0 > chunk ? 3 * na0 : chunk;
+    S.sets = 1;
+    CK(vcd_scratch(c, VCD_BUF_EENT, lists * VCD_MAX_ENTRIES * 4 + 16, &p), "coefficient lists");
+    S.ent = (uint32_t *)p;
+    // quant table (8 LODs) | meta (lists) | doubt (1 + lists) | len (all atoms or lists) | dc (all atoms)
+    size_t q_b = 8 * sizeof(vcd_quant), meta_b = lists * 4, doubt_b = (lists + 1) * 4, n_len = total_atoms > lists ? total_atoms : lists,
+           len_b = n_len * 4;
     size_t dc_b = total_atoms + 16;
     CK(vcd_scratch(c, VCD_BUF_EMETA, q_b + meta_b + doubt_b + len_b + dc_b + 64, &p), "encode metadata");
     S.qtab = (vcd_quant *)p;
     S.meta = (uint32_t *)((uint8_t *)p + q_b);
-    S.doubt = S.meta + chunk;
-    S.len = S.doubt + chunk + 1;
-    S.dc = (uint8_t *)(S.len + total_atoms);
+    S.doubt = S.meta + lists;
+    S.len = S.doubt + lists + 1;
+    S.dc = (uint8_t *)(S.len + n_len);
     CK(vcd_scratch(c, VCD_BUF_POS, (total_atoms + 1) * 8, &p), "placement");
     S.pos = (uint64_t *)p;
-    CK(vcd_scratch(c, VCD_BUF_RED, 64, &p), "totals");
+    CK(vcd_scratch(c, VCD_BUF_RED, 128, &p), "totals");
     S.red = (unsigned long long *)p;
     // keep LOD0's forward transform (128 KiB per atom) for the passes after the first when it takes at most half the
     // free memory
@@ -323,22 +332,29 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     // after the last step for a q that may still be the nearest.
     struct Visit { float q; unsigned long long bytes, present, doubt; } v[24];
     const double target = (double)info->target_ratio;
-    auto measure = [&](Visit &m, RcJob::Pass pass) -> cudaError_t {
+    auto measure = [&](Visit *m, uint32_t sets, RcJob::Pass pass) -> cudaError_t {
         cudaError_t e = cudaSuccess;
         S.size_pass = pass;
-        if (pass == RcJob::kDoubt) {   // the lists are those of the pass before
+        S.sets = sets;
+        if (pass != RcJob::kDoubt && (e = cudaMemsetAsync(S.red, 0, 24 * sets, st)) != cudaSuccess) return e;
+        if (pass != RcJob::kDoubt)
+            for (uint32_t k = 0; k < sets; ++k) set_q(S, (int)k, m[k].q);
+        if (pass == RcJob::kDoubt || sets > 1) {
+            for (uint32_t k = 0; k < sets && pass != RcJob::kDoubt; ++k)   // else the lists are those of the pass before
+                fwd_chunk(S, 0, na0, st, S.ent + k * na0 * VCD_MAX_ENTRIES, S.meta + k * na0, k);
             code_chunk(S, 0, na0, kSizes, st, S.ent, S.meta, nullptr);
         } else {
-            if ((e = cudaMemsetAsync(S.red, 0, 24, st)) != cudaSuccess) return e;
-            set_q(S, 0, m.q);
             run_range(S, 0, na0, kSizes, st, S.ent, S.meta);
         }
-        unsigned long long h[3];
-        if ((e = cudaMemcpyAsync(h, S.red, 24, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+        S.sets = 1;
+        unsigned long long h[9];
+        if ((e = cudaMemcpyAsync(h, S.red, 24 * sets, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-        m.bytes = h[0];
-        m.present = h[1];
-        m.doubt = pass == RcJob::kNear ? h[2] : 0;
+        for (uint32_t k = 0; k < sets; ++k) {
+            m[k].bytes = h[3 * k];
+            m[k].present = h[3 * k + 1];
+            m[k].doubt = pass == RcJob::kNear ? h[3 * k + 2] : 0;
+        }
         return cudaSuccess;
     };
     auto ratio = [](const Visit &m, unsigned long long more) {
@@ -349,20 +365,34 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     double best_err = INFINITY;
     uint64_t present = 0, best_bytes = 0;
     int nv = 0;
-    for (int it = 0; it < (info->fixed_q ? 0 : 24); ++it) {
-        uint32_t mid = lo + (hi - lo) / 2;
-        Visit &m = v[nv];
-        m.q = f_of(mid);
-        CK(measure(m, RcJob::kNear), "rate control pass");
-        present = m.present;
+    const int steps = info->fixed_q ? 0 : 24;
+    while (nv < steps) {
+        // Once the transform is kept, a step of few atoms takes as long with three
+        // quantisers as with one: its own and both that the next step may come to
+        // (540 atoms: 0.26 and 0.25 ms). Not in the first steps, where one of those
+        // is a much finer one than either step needs.
+        const uint32_t mid = lo + (hi - lo) / 2;
+        const uint32_t sets = three && S.coef_valid && nv >= 3 && nv + 1 < steps ? 3 : 1;
+        Visit m[3];
+        m[0].q = f_of(mid);
+        m[1].q = f_of(mid + (hi - mid) / 2);   // after lo = mid
+        m[2].q = f_of(lo + (mid - lo) / 2);    // after hi = mid
+        CK(measure(m, sets, RcJob::kNear), "rate control pass");
+        present = m[0].present;
         if (present == 0) break;
-        // the doubt of a pass this near is likely to matter, and its lists are at hand
-        const double want = (double)(32768ull * m.present) / target;
-        if ((ratio(m, m.doubt) < target) != (ratio(m, 0) < target) ||
-            fabs((double)m.bytes - want) <= 4.0 * (double)m.doubt)
-            if (m.doubt) CK(measure(m, na0 <= kChunk ? RcJob::kDoubt : RcJob::kExact), "rate control pass");
-        if (ratio(m, 0) < target) lo = mid; else hi = mid;
-        ++nv;
+        for (uint32_t k = 0, end = 0; !end;) {
+            // the doubt of a pass this near is likely to matter, and its lists are at hand
+            const double want = (double)(32768ull * m[k].present) / target;
+            if (m[k].doubt && ((ratio(m[k], m[k].doubt) < target) != (ratio(m[k], 0) < target) ||
+                               fabs((double)m[k].bytes - want) <= 4.0 * (double)m[k].doubt))
+                CK(measure(m, sets, na0 <= kChunk ? RcJob::kDoubt : RcJob::kExact), "rate control pass");
+            const uint32_t at = b_of(m[k].q);
+            const bool below = ratio(m[k], 0) < target;
+            if (below) lo = at; else hi = at;
+            v[nv++] = m[k];
+            end = k || sets == 1;
+            k = below ? 1 : 2;
+        }
     }
     auto consider = [&](const Visit &m) {
         const double err = fabs(ratio(m, 0) - target);
@@ -383,7 +413,7 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
             if (v[i].doubt && e <= near_err) near = i, near_err = e;
         }
         if (near < 0) break;
-        CK(measure(v[near], RcJob::kExact), "rate control pass");
+        CK(measure(&v[near], 1, RcJob::kExact), "rate control pass");
         consider(v[near]);
     }
     S.size_pass = RcJob::kExact;
