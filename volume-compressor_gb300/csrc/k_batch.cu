@@ -123,14 +123,38 @@ __global__ void k_ua_scatter(BatchJob J) {
     }
 }
 
-__global__ void __launch_bounds__(kLaneThreads) k_rc_batch_lanes(BatchJob J) {
+template <bool SOLO>
+__global__ void __launch_bounds__(SOLO ? kLaneCta : kLaneThreads) k_rc_batch_lanes(BatchJob J) {
+    extern __shared__ __align__(16) uint8_t stage[];
     __shared__ uint32_t bstart[10];   // the band table and a copy of its end (RcLane)
     __shared__ uint32_t S[kLaneWarps][kLaneRows * 32];
     if (threadIdx.x < 10) bstart[threadIdx.x] = J.band_start[threadIdx.x < 9 ? threadIdx.x : 8];
     __syncthreads();
     const uint32_t n_present = J.sort_ctl[kSortBuckets];   // 0 when the scalar kernel decodes this batch
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t i = 32u * lane_warp_rank(J.sms) + lane;
+    const uint32_t alone = SOLO ? lane_solo(n_present, J.sms) : 0u;
+    if constexpr (SOLO) if (threadIdx.x >= kLaneThreads) {
+        const uint32_t s = lane_solo_rank(J.sms);
+        if (s >= alone) return;
+        const uint32_t u = J.order[s];
+        const vcd_atom e = J.atoms[J.ua[u].idx];
+        uint32_t cap = 8u * (e.len - 1u) + 64u, n = 0;
+        if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
+        uint32_t *dst = J.ent + J.ent_off[u];
+        const int bad = solo_decode(stage + ((threadIdx.x >> 5) - kLaneWarps) * kSoloStage, J.arc + e.off + 1, e.len - 1u,
+                                    bstart, [&](uint32_t p, uint32_t lv) {
+                                        if (n < cap) dst[n] = p | (lv << 16);
+                                        ++n;
+                                    });
+        if (lane) return;
+        J.cnt[u] = (n > cap ? cap : n) | (n > cap ? kEntOverflow : 0u) | (bad ? kEntBad : 0u);
+        if (bad) {
+            const UAtom a = J.ua[u];
+            for (uint32_t d = a.dst_begin; d < a.dst_end; ++d) atomicOr(J.req_err + J.dst[d], 1u);
+        }
+        return;
+    }
+    const uint32_t i = alone + 32u * lane_warp_rank(J.sms) + lane;
     const bool active = i < n_present;
     uint32_t u = 0, cap = 0;
     vcd_atom e = {};
@@ -399,7 +423,11 @@ static void launch_rc(const BatchJob &J, int num_sms, uint32_t max_ua, cudaStrea
         k_ua_hist<<<sg, 256, 0, s>>>(J);
         launch_len_scan(J.sort_ctl, s);
         k_ua_scatter<<<sg, 256, 0, s>>>(J);
-        k_rc_batch_lanes<<<lane_grid(max_ua < 1 ? 1 : max_ua, (uint32_t)num_sms), kLaneThreads, 0, s>>>(J);
+        // a batch may hold half its capacity: solo warps wherever their CTAs, two an SM, all fit at once
+        smem_attr((const void *)k_rc_batch_lanes<true>, (int)kSoloSmem);
+        const unsigned lg = lane_grid(max_ua < 1 ? 1 : max_ua, (uint32_t)num_sms);
+        if (max_ua <= 64u * 4u * (uint32_t)num_sms) k_rc_batch_lanes<true><<<lg, kLaneCta, kSoloSmem, s>>>(J);
+        else k_rc_batch_lanes<false><<<lg, kLaneThreads, 0, s>>>(J);
     }
     // capacity within the latency decoder's range: stage the streams (one CTA
     // per SM at most, with a warp per atom)

@@ -221,14 +221,38 @@ __global__ void k_len_scatter(DecodeJob J) {
 
 static_assert(kSortBuckets == 4 * 1024, "k_len_scan: 1024 threads x 4 counters");
 
-__global__ void __launch_bounds__(kLaneThreads) k_rc_lanes(DecodeJob J, uint32_t sms) {
+template <bool SOLO>
+__global__ void __launch_bounds__(SOLO ? kLaneCta : kLaneThreads) k_rc_lanes(DecodeJob J, uint32_t sms) {
+    extern __shared__ __align__(16) uint8_t stage[];
     __shared__ uint32_t bstart[10];   // the band table and a copy of its end (RcLane)
     __shared__ uint32_t S[kLaneWarps][kLaneRows * 32];
     if (threadIdx.x < 10) bstart[threadIdx.x] = J.band_start[threadIdx.x < 9 ? threadIdx.x : 8];
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t i = 32ull * lane_warp_rank(sms) + lane;
-    const bool active = i < J.sort_ctl[kSortBuckets];
+    const uint32_t n_present = J.sort_ctl[kSortBuckets], alone = SOLO ? lane_solo(n_present, sms) : 0u;
+    if constexpr (SOLO) if (threadIdx.x >= kLaneThreads) {
+        const uint32_t s = lane_solo_rank(sms);
+        if (s >= alone) return;
+        const uint64_t t = J.order[s];
+        uint32_t az, ay, ax;
+        box_atom(J, t, az, ay, ax);
+        const vcd_atom e = J.atoms[job_atom(J, t, az, ay, ax)];
+        uint32_t cap = 8u * (e.len - 1u) + 64u, n = 0;
+        if (e.len - 1u > VCD_MAX_ENTRIES / 8u || cap > VCD_MAX_ENTRIES) cap = VCD_MAX_ENTRIES;
+        uint32_t *dst = J.ent + J.ent_off[t];
+        const int bad = solo_decode(stage + ((threadIdx.x >> 5) - kLaneWarps) * kSoloStage, J.arc + e.off + 1, e.len - 1u,
+                                    bstart, [&](uint32_t p, uint32_t lv) {
+                                        if (n < cap) dst[n] = p | (lv << 16);
+                                        ++n;
+                                    });
+        if (lane) return;
+        J.cnt[t] = (n > cap ? cap : n) | (n > cap ? kEntOverflow : 0u) | (bad ? kEntBad : 0u);
+        atomicAdd(J.nnz_total, (unsigned long long)(n > cap ? cap : n));
+        if (bad) atomicMin(J.err, (uint32_t)(t < 0xFFFFFFFFull ? t : 0xFFFFFFFEull));
+        return;
+    }
+    const uint64_t i = alone + 32ull * lane_warp_rank(sms) + lane;
+    const bool active = i < n_present;
     uint64_t t = 0;
     vcd_atom e = {};
     uint32_t cap = 0;
@@ -349,7 +373,13 @@ static void launch_rc(const DecodeJob &J, int num_sms, cudaStream_t s, const Sta
             Jl.sort_ctl = J.sort_ctl + 2;   // Jl.sort_ctl[kSortBuckets]: the per-lane count
         }
         const unsigned lane_blocks = lane_grid(J.n_atoms - ns, (uint32_t)num_sms);
-        if (lane_blocks) k_rc_lanes<<<lane_blocks, kLaneThreads, 0, s>>>(Jl, (uint32_t)num_sms);   // (0: every atom solo)
+        smem_attr((const void *)k_rc_lanes<true>, (int)kSoloSmem);
+        if (!lane_blocks) {   // every atom solo on the second stream
+        } else if (lane_solo((uint32_t)(J.n_atoms < 0xFFFFFFFFull ? J.n_atoms : 0xFFFFFFFFull), (uint32_t)num_sms)) {
+            k_rc_lanes<true><<<lane_blocks, kLaneCta, kSoloSmem, s>>>(Jl, (uint32_t)num_sms);
+        } else {
+            k_rc_lanes<false><<<lane_blocks, kLaneThreads, 0, s>>>(Jl, (uint32_t)num_sms);
+        }
         if (ns) cudaStreamWaitEvent(s, ev->join, 0);
         return;
     }

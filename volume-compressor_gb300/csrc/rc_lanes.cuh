@@ -19,6 +19,42 @@ namespace vcg {
 constexpr uint32_t kLaneWarps = 8;
 constexpr int kLaneThreads = 32 * kLaneWarps;
 
+// Four more warps, one per sub-partition, take the longest atoms alone where the
+// others fill at most one warp of lanes a sub-partition: a lane's decision takes
+// two to three times as long as a lone atom's, so the longest atoms set the time,
+// and there the sub-partition has issue slots left. Beside two warps of lanes it
+// has not: 32,768 atoms take 6.40 ms with them and 5.56 without, 10,846 at target
+// 50 1.52 and 1.83, 16,969 of four LODs at target 20 5.01 and 6.73.
+constexpr uint32_t kSoloWarps = 4;
+constexpr int kLaneCta = kLaneThreads + 32 * kSoloWarps;
+constexpr uint32_t kSoloStage = 22u * 1024u;                 // stream bytes such a warp stages in shared memory
+constexpr uint32_t kSoloSmem = kSoloWarps * kSoloStage;      // two CTAs of it fit an SM
+
+// how many of n atoms run alone
+__host__ __device__ inline uint32_t lane_solo(uint32_t n, uint32_t sms) {
+    const uint32_t k = kSoloWarps * sms;
+    return n > 32u * 4u * sms ? 0u : n < k ? n : k;
+}
+
+// the place in the payload-length order of the calling warp's atom, one of the
+// solo warps of the first `sms` CTAs (else past every atom)
+__device__ __forceinline__ uint32_t lane_solo_rank(uint32_t sms) {
+    return blockIdx.x < sms ? ((threadIdx.x >> 5) - kLaneWarps) * sms + blockIdx.x : 0xFFFFFFFFu;
+}
+
+// The whole warp calls this: lane 0 decodes the stream and returns 1 for a
+// malformed one; the others return at once.
+template <class Sink>
+__device__ __forceinline__ int solo_decode(uint8_t *stage, const uint8_t *src, uint32_t len, const uint32_t *bstart,
+                                           Sink &&sink) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool fits = len + kStagePad <= kSoloStage;
+    if (fits) stage_stream(stage, src, len, lane);
+    __syncwarp();
+    if (lane) return 0;
+    return fits ? rc_decode_levels_sm(stage, len, bstart, sink) : rc_decode_levels_lat(src, len, bstart, sink);
+}
+
 inline unsigned lane_grid(uint64_t n_atoms, uint32_t sms) {
     const uint64_t warps = (n_atoms + 31) / 32, per = (uint64_t)kLaneWarps * sms;
     return (unsigned)((warps + per - 1) / per * sms);
