@@ -26,7 +26,9 @@ namespace vcg {
 
 // k_fwd holds an atom's tile and levels, so an SM runs one CTA: 16 warps of it,
 // two rows or lines a thread, hide each other's latency (the 37,451 atoms of a
-// 1024^3 pyramid in 6.9 ms; 8 warps and the transform kept for later passes, 8.7).
+// 1024^3 pyramid in 6.3 ms; 8 warps and the transform kept for later passes, 8.7).
+// The integer pipes bound it: multiplies of the passes, then the quantiser's
+// arithmetic, which groups without a level skip.
 constexpr int kFwdThreads = 512;
 constexpr int kQuantThreads = 256;
 constexpr size_t kFwdSmem = kTileBytes + 32768 * sizeof(int16_t);
@@ -49,33 +51,39 @@ __device__ __forceinline__ void load_row(const uint8_t *vol, uint32_t nx, uint32
     for (uint32_t i = 0; i < cnt; ++i) w[i >> 2] |= (uint32_t)__ldg(p + i) << (8 * (i & 3));
 }
 
-// Quantiser class of raster r: its frequency, + 94 where the alternate step
-// applies (src/vc/vc.c:273-279, 293-306).
-__device__ __forceinline__ uint32_t quant_class(uint32_t r, const uint32_t *alt) {
-    const uint32_t f = (r >> 10) + ((r >> 5) & 31u) + (r & 31u);
-    return f + 94u * ((alt[r >> 5] >> (r & 31u)) & 1u);
-}
-
 // A coefficient with its class, as the quantiser needs it: |cf| in bits 0-16
 // (the transform of 8-bit voxels about a centre in [0, 255] reaches at most
 // 46,132, the DC of a block 255 away from its centre), the class in bits 17-24,
 // the sign in bit 31. Quantising it needs no scan order or class lookup.
-__device__ __forceinline__ uint32_t coef_pack(int32_t cf, uint32_t r, const uint32_t *alt) {
+__device__ __forceinline__ uint32_t coef_pack(int32_t cf, uint32_t cls) {
     const uint32_t mag = cf < 0 ? 0u - (uint32_t)cf : (uint32_t)cf;
-    return mag | (quant_class(r, alt) << 17) | (cf < 0 ? 0x80000000u : 0u);
+    return mag | (cls << 17) | ((uint32_t)cf & 0x80000000u);
 }
+
+// Quantiser constants of an atom's q by class. A magnitude of at least `least`
+// has a level: the smallest whole number not below the dead zone dz.
+struct QuantShared {
+    uint32_t least[VCD_NCLASS];
+    float dz[VCD_NCLASS], rr[VCD_NCLASS];
+    __device__ __forceinline__ void load(const vcd_quant &q) {
+        for (int i = threadIdx.x; i < VCD_NCLASS; i += blockDim.x) {
+            dz[i] = q.dz[i];
+            rr[i] = q.rr[i];
+            least[i] = (uint32_t)__float2int_ru(fminf(fmaxf(q.dz[i], 0.0f), 1e9f));
+        }
+    }
+    __device__ __forceinline__ bool has(uint32_t w) const { return (w & 0x1FFFFu) >= least[(w >> 17) & 0xFFu]; }
+};
 
 // Dead-zone quantiser of a packed coefficient, as the release build evaluates
 // it (src/vc/vc.c:293-306): level = trunc((|cf| - dz) r' + 1) for |cf| >= dz,
 // clamped, with the coefficient's sign.
-__device__ __forceinline__ int32_t quant_packed(uint32_t w, const float *qdz, const float *qrr) {
+__device__ __forceinline__ int32_t quant_packed(uint32_t w, const QuantShared &q) {
     const uint32_t cls = (w >> 17) & 0xFFu;
     const float fa = __int2float_rn((int32_t)(w & 0x1FFFFu));
-    int32_t level = 0;
-    if (fa >= qdz[cls]) {
-        level = __float2int_rz(__fadd_rn(__fmul_rn(__fsub_rn(fa, qdz[cls]), qrr[cls]), 1.0f));
-        if (level > 32767) level = 32767;
-    }
+    int32_t level = __float2int_rz(__fadd_rn(__fmul_rn(__fsub_rn(fa, q.dz[cls]), q.rr[cls]), 1.0f));
+    if (level > 32767) level = 32767;
+    level = q.has(w) ? level : 0;
     return (w >> 31) ? -level : level;
 }
 
@@ -87,8 +95,8 @@ __device__ __forceinline__ int32_t quant_packed(uint32_t w, const float *qdz, co
 // pass 2 places each lane's entries after a warp prefix sum of the per-lane
 // counts, skipping groups without a nonzero level.
 template <int NT, class Pk4>
-__device__ __forceinline__ uint32_t quant_compact(Pk4 &&pk4, const float *qdz, const float *qrr, int16_t *lv,
-                                                  uint32_t *wcnt, uint32_t *dst) {
+__device__ __forceinline__ uint32_t quant_compact(Pk4 &&pk4, const QuantShared &q, int16_t *lv, uint32_t *wcnt,
+                                                  uint32_t *dst) {
     constexpr uint32_t kPer = 32768 / (NT / 32);
     static_assert(kPer % 512 == 0, "whole groups of loads");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -104,11 +112,16 @@ __device__ __forceinline__ uint32_t quant_compact(Pk4 &&pk4, const float *qdz, c
         for (uint32_t g = 0; g < kG; ++g) w[g] = pk4(p0 + i + 128 * g);
 #pragma unroll
         for (uint32_t g = 0; g < kG; ++g) {
-            const int32_t l0 = quant_packed(w[g].x, qdz, qrr), l1 = quant_packed(w[g].y, qdz, qrr);
-            const int32_t l2 = quant_packed(w[g].z, qdz, qrr), l3 = quant_packed(w[g].w, qdz, qrr);
-            *reinterpret_cast<uint2 *>(lv + p0 + i + 128 * g) =
-                make_uint2((uint32_t)(uint16_t)l0 | ((uint32_t)l1 << 16), (uint32_t)(uint16_t)l2 | ((uint32_t)l3 << 16));
-            cnt += (uint32_t)(l0 != 0) + (uint32_t)(l1 != 0) + (uint32_t)(l2 != 0) + (uint32_t)(l3 != 0);
+            uint2 out = make_uint2(0u, 0u);
+            // most groups of the upper bands have no level at all
+            if (__any_sync(0xFFFFFFFFu, q.has(w[g].x) || q.has(w[g].y) || q.has(w[g].z) || q.has(w[g].w))) {
+                const int32_t l0 = quant_packed(w[g].x, q), l1 = quant_packed(w[g].y, q);
+                const int32_t l2 = quant_packed(w[g].z, q), l3 = quant_packed(w[g].w, q);
+                out = make_uint2((uint32_t)(uint16_t)l0 | ((uint32_t)l1 << 16),
+                                 (uint32_t)(uint16_t)l2 | ((uint32_t)l3 << 16));
+                cnt += (uint32_t)(l0 != 0) + (uint32_t)(l1 != 0) + (uint32_t)(l2 != 0) + (uint32_t)(l3 != 0);
+            }
+            *reinterpret_cast<uint2 *>(lv + p0 + i + 128 * g) = out;
         }
     }
     cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
@@ -149,12 +162,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
     extern __shared__ int32_t smem[];
     int32_t *T = smem;                                          // the padded atom tile (dct32.cuh)
     int16_t *L = reinterpret_cast<int16_t *>(smem + kTileInts); // levels in scan order
-    __shared__ float qdz[VCD_NCLASS], qrr[VCD_NCLASS];
-    __shared__ uint32_t alt[1024];
+    __shared__ QuantShared q;
     __shared__ uint32_t red[32];
     __shared__ uint32_t wcnt[kFwdThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < 1024; i += kFwdThreads) alt[i] = J.alt_mask[i];
     int cur_lod = -1;
 
     for (uint64_t t = blockIdx.x; t < J.n_atoms; t += gridDim.x) {
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
         const int qi = J.qsel ? (int)J.qsel[t] : lod;
         if (qi != cur_lod) {   // uniform across the CTA: quantiser constants of this atom
             __syncthreads();   // every thread is done with the previous constants
-            for (int i = tid; i < VCD_NCLASS; i += kFwdThreads) { qdz[i] = J.q[qi].dz[i]; qrr[i] = J.q[qi].rr[i]; }
+            q.load(J.q[qi]);
             cur_lod = qi;
             __syncthreads();
         }
@@ -183,7 +194,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
             }
             dc = (int32_t)(dcz & 0xFFu);
             total = quant_compact<kFwdThreads>(
-                [&](uint32_t p) { return __ldcs(reinterpret_cast<const uint4 *>(cptr + p)); }, qdz, qrr, L, wcnt, dst);
+                [&](uint32_t p) { return __ldcs(reinterpret_cast<const uint4 *>(cptr + p)); }, q, L, wcnt, dst);
         } else {
             const uint8_t *vol = J.vol[lod];
             const uint32_t nx = J.dims[lod][0], ny = J.dims[lod][1], nz = J.dims[lod][2];
@@ -251,14 +262,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd(FwdJob J) {
             }
             __syncthreads();
             auto tile = [&](uint32_t p) {
-                const uint2 sc = __ldg(reinterpret_cast<const uint2 *>(J.scan + p));
-                const uint32_t r0 = sc.x & 0xFFFFu, r1 = sc.x >> 16, r2 = sc.y & 0xFFFFu, r3 = sc.y >> 16;
-                const uint4 w = make_uint4(coef_pack(T[tile_idx(r0)], r0, alt), coef_pack(T[tile_idx(r1)], r1, alt),
-                                           coef_pack(T[tile_idx(r2)], r2, alt), coef_pack(T[tile_idx(r3)], r3, alt));
+                const uint4 at = __ldg(reinterpret_cast<const uint4 *>(J.place + p));
+                auto get = [&](uint32_t a) { return coef_pack(T[a & 0xFFFFu], a >> 16); };
+                const uint4 w = make_uint4(get(at.x), get(at.y), get(at.z), get(at.w));
                 if (cached) *reinterpret_cast<uint4 *>(cptr + p) = w;   // kept in scan order
                 return w;
             };
-            total = quant_compact<kFwdThreads>(tile, qdz, qrr, L, wcnt, dst);
+            total = quant_compact<kFwdThreads>(tile, q, L, wcnt, dst);
         }
         if (tid == 0) J.meta[t] = total | ((uint32_t)dc << 16);
     }
@@ -270,10 +280,10 @@ constexpr size_t kQuantSmem = 32768 * sizeof(int16_t);
 
 __global__ void __launch_bounds__(kQuantThreads) k_quant_cached(FwdJob J) {
     extern __shared__ int16_t lv[];
-    __shared__ float qdz[VCD_NCLASS], qrr[VCD_NCLASS];
+    __shared__ QuantShared q;
     __shared__ uint32_t wcnt[kQuantThreads / 32];
     const int tid = threadIdx.x;
-    for (int i = tid; i < VCD_NCLASS; i += kQuantThreads) { qdz[i] = J.q[0].dz[i]; qrr[i] = J.q[0].rr[i]; }
+    q.load(J.q[0]);
     __syncthreads();
     for (uint64_t t = blockIdx.x; t < J.n_atoms; t += gridDim.x) {
         const uint64_t ca = J.first + t;
@@ -284,7 +294,7 @@ __global__ void __launch_bounds__(kQuantThreads) k_quant_cached(FwdJob J) {
         }
         const uint32_t *cptr = J.coef + ca * 32768ull;
         const uint32_t total = quant_compact<kQuantThreads>(
-            [&](uint32_t p) { return __ldcs(reinterpret_cast<const uint4 *>(cptr + p)); }, qdz, qrr, lv, wcnt,
+            [&](uint32_t p) { return __ldcs(reinterpret_cast<const uint4 *>(cptr + p)); }, q, lv, wcnt,
             J.ent + t * (uint64_t)VCD_MAX_ENTRIES);
         if (tid == 0) J.meta[t] = total | ((dcz & 0xFFu) << 16);
     }
@@ -506,8 +516,15 @@ void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s) {
     k_fwd<<<(unsigned)grid, kFwdThreads, kFwdSmem, s>>>(J);
 }
 
-void enc_costs(EncCosts *t) {
-    memset(t, 0, sizeof *t);
+void enc_tables(EncTables *et, const vcd_tables *vt) {
+    memset(et, 0, sizeof *et);
+    for (uint32_t p = 0; p < 32768; ++p) {
+        const uint32_t r = vt->scan[p], f = (r >> 10) + ((r >> 5) & 31u) + (r & 31u);
+        // the alternate step's class where it applies (src/vc/vc.c:273-279, 293-306)
+        const uint32_t cls = f + 94u * ((vt->alt_mask[r >> 5] >> (r & 31u)) & 1u);
+        et->place[p] = (r >> 10) * kSlabPitch + ((r >> 5) & 31u) * kRowPitch + (r & 31u) | cls << 16;
+    }
+    EncCosts *t = &et->costs;
     const double bit = kCostOne, e = 4096.0 / 16777216.0 * 1.4427 * 1.0001;   // log2(e) and the square term, above
     for (uint32_t c = 1; c < 4096; ++c)
         t->one[c] = make_uint2((uint32_t)llround((12.0 - log2((double)c)) * bit),

@@ -46,8 +46,7 @@ struct FwdJob {
     uint64_t n_atoms;
     const vcd_quant *q;          // per-LOD quantiser constants (device, [lod])
     const uint8_t *qsel;         // optional: per atom (this launch) index into q instead of its LOD
-    const uint16_t *scan;        // scan position -> raster index
-    const uint32_t *alt_mask;
+    const uint32_t *place;       // scan position -> index in the transform's tile | quantiser class << 16 (EncTables)
     uint32_t *ent;               // per atom VCD_MAX_ENTRIES slots: scan position | level << 16
     uint32_t *meta;              // per atom
     // coefficient cache of canonical atoms [0, coef_n): 32768 packed words per
@@ -108,7 +107,8 @@ void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s);
 // atoms that are all LOD0 with kept coefficients: quantise and compact only
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s);
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s);
-void enc_costs(EncCosts *t);   // the table, on the host
+struct EncTables;
+void enc_tables(EncTables *t, const vcd_tables *vt);   // on the host
 // atoms that a pass for lengths takes as sets, or at once four a CTA, at most
 uint64_t size_sets_atoms(int num_sms);
 // atoms that a coder pass runs as groups at most

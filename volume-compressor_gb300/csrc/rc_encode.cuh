@@ -583,6 +583,12 @@ struct EncCosts {
     uint2 eight[4096];   // [q]: eight zeros from q = 4096 - p: cost, error << 16 | q after them
 };
 
+// The encoder's tables on the device.
+struct EncTables {
+    EncCosts costs;
+    uint32_t place[32768];   // scan position -> index in the forward transform's tile | quantiser class << 16
+};
+
 #ifdef __CUDACC__
 struct EncSize {   // least and most bits are cost - lo and cost + hi
     uint64_t cost;

@@ -51,17 +51,17 @@ static void init_once(void) {
         free(t);
         return;
     }
+    EncTables *et = (EncTables *)malloc(sizeof(EncTables));
+    if (et) enc_tables(et, t);
     free(t);
-    EncCosts *ec = (EncCosts *)malloc(sizeof(EncCosts));
-    if (!ec) { snprintf(g_err, sizeof g_err, "cost table: out of memory"); return; }
-    enc_costs(ec);
-    if ((e = cudaMalloc(&g_dev.costs, sizeof(EncCosts))) != cudaSuccess ||
-        (e = cudaMemcpy(g_dev.costs, ec, sizeof(EncCosts), cudaMemcpyHostToDevice)) != cudaSuccess) {
-        vcd_set_error("cost table upload", e);
-        free(ec);
+    if (!et) { snprintf(g_err, sizeof g_err, "encoder tables: out of memory"); return; }
+    if ((e = cudaMalloc(&g_dev.enc, sizeof(EncTables))) != cudaSuccess ||
+        (e = cudaMemcpy(g_dev.enc, et, sizeof(EncTables), cudaMemcpyHostToDevice)) != cudaSuccess) {
+        vcd_set_error("encoder table upload", e);
+        free(et);
         return;
     }
-    free(ec);
+    free(et);
     __atomic_store_n(&g_init_rc, 0, __ATOMIC_RELEASE);
 }
 

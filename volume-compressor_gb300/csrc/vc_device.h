@@ -65,7 +65,7 @@ struct vcd_archive {
 struct vcd_device {
     int device, num_sms;
     vcd_tables *tables;          // device copy
-    void *costs;                 // device copy of the encoder's EncCosts
+    void *enc;                   // device copy of the encoder's EncTables
     uint32_t band_start[9];
 };
 

@@ -18,6 +18,8 @@ using namespace vcg;
 
 static const uint64_t kChunk = 32768;   // atoms per forward/coder launch (4 GiB of list scratch)
 
+static const EncTables *enc_dev() { return (const EncTables *)g_dev.enc; }
+
 static inline float f_of(uint32_t b) { float f; memcpy(&f, &b, 4); return f; }
 static inline uint32_t b_of(float f) { uint32_t b; memcpy(&b, &f, 4); return b; }
 
@@ -104,8 +106,7 @@ static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uin
     F.first = c0;
     F.n_atoms = n;
     F.q = S.qtab + set;
-    F.scan = g_dev.tables->scan;
-    F.alt_mask = g_dev.tables->alt_mask;
+    F.place = enc_dev()->place;
     F.ent = ent;
     F.meta = meta;
     F.coef = S.coef;
@@ -142,7 +143,7 @@ static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaS
     if (pass == kSizes) {
         R.n_atoms = n * S.sets;
         R.per = n;
-        R.costs = (const EncCosts *)g_dev.costs;
+        R.costs = &enc_dev()->costs;
         R.doubt = meta == S.meta ? S.doubt : S.doubt2;
         R.pass = S.size_pass;
         R.totals = S.red;
@@ -591,8 +592,7 @@ extern "C" int vcd_encode_segments(const vcd_seg *segs, int nseg, const float *q
             F.n_atoms = n;
             F.q = qtab;
             F.qsel = dqsel;
-            F.scan = g_dev.tables->scan;
-            F.alt_mask = g_dev.tables->alt_mask;
+            F.place = enc_dev()->place;
             F.ent = ent;
             F.meta = dmeta;
             launch_fwd(F, g_dev.num_sms, st);
