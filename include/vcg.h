@@ -35,8 +35,8 @@ typedef struct {
 vc_status vcg_decode_regions(vc_archive *a, uint32_t n, const vcg_region_request *reqs, int out_on_device,
                              vc_status *status);
 // Launch shape the calling thread uses (0 before its first batch): range-decoder
-// policy (warps per SM sub-partition that decode one atom each before atoms
-// share warps in lockstep; see vcg_set_rc_scalar_warps), transform CTA size
+// policy (warps per SM sub-partition that decode one atom each before every
+// lane takes an atom; see vcg_set_rc_scalar_warps), transform CTA size
 // (32 x warps per atom) and transform form (0 butterfly on the CUDA cores,
 // 1 int8 tensor cores). The autotuner times every combination on the process's
 // first batch; all give identical bytes.
@@ -53,7 +53,8 @@ vc_status vcg_set_batch_shape(int rc_scalar_warps, int transform_threads, int tr
 // one-atom decoder, longest payloads first above one per sub-partition, on a
 // copy of its stream in shared memory where the streams fit; above that the
 // per-lane decoder (every lane of a warp decodes its own atom, atoms in order
-// of payload length). w = 0: no atom keeps a warp to itself (above one atom
+// of payload length; up to 32 atoms per sub-partition the longest four per SM
+// have warps of their own). w = 0: no atom keeps a warp to itself (above one atom
 // per sub-partition the per-lane decoder, below it atoms share warps in
 // lockstep); w < 0 restores the default (8: measured on GB300, the per-lane
 // decoder wins from about 4,000 atoms on, depending on the atoms' sizes).

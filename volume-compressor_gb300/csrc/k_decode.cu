@@ -5,8 +5,9 @@
 //   k_scan_u64   one CTA: exclusive scan of the capacities (list placement)
 //   k_rc_decode  one thread per PRESENT atom: serial range decode of its
 //                payload into (scan position, level) pairs (src/vc/vc.c:545-560);
-//                one atom per warp for small decodes, a warp of atoms in
-//                lockstep for large ones
+//                one atom per warp for small decodes
+//   k_rc_lanes   the same for large ones: one atom per lane, the longest of
+//                a middling one alone in a warp
 //   k_idct       persistent, one CTA per SM: levels dequantised
 //                (src/vc/vc.c:327-338), inverse passes along x, y, z on the tensor
 //                cores (idct_mma.cuh), dc added, clamped, cropped into the box
@@ -280,14 +281,10 @@ __global__ void __launch_bounds__(SOLO ? kLaneCta : kLaneThreads) k_rc_lanes(Dec
 // each get a warp of their own whose lane 0 runs the latency decoder, on a
 // second stream beside k_rc_lanes, which takes the atoms after them. The
 // longest atoms set the per-lane decoder's time (every lane steps at about the
-// same pace, whatever its atom, bound by its own dependency chain), and the
-// latency decoder's chain is about twice as fast per decision while its one
-// lane takes about a third of a sub-partition's issue slots. Off by default
-// (vcg_set_rc_solo): measured on GB300 (1024^3 at target 10, range decode
-// 8.26 ms without) it gave 7.88 ms with 76 solo atoms in one process and
-// 8.41 ms in another, 8.0-8.3 ms with 152-608, and once 15.4 ms when the two
-// kernels ran one after the other: the gain depends on where the solo warps
-// land.
+// same pace, whatever its atom, bound by its own dependency chain). Off by
+// default (vcg_set_rc_solo): where the solo warps land is the hardware's choice,
+// and a second kernel may run after the first instead of beside it. Where it
+// pays, k_rc_lanes has solo warps of its own (lane_solo).
 __global__ void __launch_bounds__(32) k_rc_solo(DecodeJob J, uint32_t n) {
     __shared__ uint32_t bstart[9];
     if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];

@@ -109,9 +109,10 @@ struct BatchShape {              // tunables the autotuner chooses among
 // above that the plain decode path runs the per-lane decoder (k_rc_lanes: all
 // 32 lanes of a warp, each its own atom; at target 10 it takes 4.6 ms from a
 // thousand to ten thousand atoms, where the one-atom decoder goes from 2.5 ms at
-// 608 over 3.9 at 3,072 to 4.9 at 4,864). The batched path still runs the lockstep
-// decoder for G > 1: the fewest warps per sub-partition k that keep a warp at
-// 32 atoms or fewer, the atoms spread evenly over k warps per sub-partition.
+// 608 over 3.9 at 3,072 to 4.9 at 4,864). Without an
+// order buffer the lockstep decoder serves G > 1: the fewest warps per
+// sub-partition k that keep a warp at 32 atoms or fewer, the atoms spread evenly
+// over k warps per sub-partition.
 __host__ __device__ inline uint32_t rc_lanes_for(uint64_t n_atoms, uint32_t sms, uint32_t scalar_warps) {
     const uint64_t slots = 4ull * sms;
     if (n_atoms <= (uint64_t)scalar_warps * slots) return 1;

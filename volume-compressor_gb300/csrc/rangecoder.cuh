@@ -1,6 +1,7 @@
 // Adaptive binary range coder and coefficient context coder (device): one
-// atom per GPU thread, either alone in its warp (latency path) or in a warp of
-// atoms decoded in lockstep (throughput path).
+// atom per GPU thread, alone in its warp (few atoms) or a lane of it (many). The
+// encoders that a launch runs are in rc_encode.cuh; the lockstep one here writes
+// the atoms whose sums outgrow their slot.
 //
 // Bit-exact with the reference's coder (src/vc/vc.c:344-560): 12-bit P(0),
 // shift-5 adaptation, LZMA-style carry-less low with a cached byte, 16-bit EOB
@@ -653,7 +654,8 @@ struct RcLane {
 
 // ---------------------------------------------------------------- latency decoder
 // One atom on one lane when few atoms share the GPU, so that the dependency
-// chain of one decision is all that counts: both outcomes of a decision (the
+// chain of one decision is all that counts, and whose stream does not fit
+// rc_decode_levels_sm's shared memory: both outcomes of a decision (the
 // new range renormalised, the adapted probability) are computed before the
 // compare, which then only selects; the byte fetch is predicated, not
 // branched; and a significance decision takes one branch (a one, or the end of

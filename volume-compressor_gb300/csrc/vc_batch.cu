@@ -2,8 +2,8 @@
 // atoms, their destination lists, the request boxes, list offsets) into
 // grow-only device buffers, then replay one CUDA graph of the persistent
 // range-decode + transform launches. The launch shape (range-decoder policy:
-// warps per SM sub-partition that decode one atom each before atoms share warps
-// in lockstep; transform on the CUDA cores with 8 or 16 warps per atom, or on
+// warps per SM sub-partition that decode one atom each before every lane takes
+// an atom; transform on the CUDA cores with 8 or 16 warps per atom, or on
 // the int8 tensor cores) is picked once per process by timing every candidate on
 // the first batch (all candidates produce identical bytes); threads that start
 // later take the tuned shape.
