@@ -432,32 +432,52 @@ __global__ void __launch_bounds__(32 * kLanesWarps) k_rc_encode_lanes(RcJob J, u
     if (t < J.n_atoms) J.len[t] = on ? n + 1u : 0u;
 }
 
-// A warp per atom: [dc] and the coder bytes.
+// Where the payload of atom t goes.
+__device__ __forceinline__ uint8_t *resolve_dst(const ResolveJob &J, uint64_t t) {
+    if (J.dst_off) return J.arc + J.dst_off[t];
+    const uint64_t a = J.canon_first + t;   // canonical index
+    return J.arc + J.pos[a] + (J.lay.first_in_region(a) ? kL2Bytes : 0ull);
+}
+
+// A warp per atom: [dc] and the coder bytes; atoms with more sums than their slot
+// holds are collected for k_rc_encode_rest.
 __global__ void __launch_bounds__(256) k_resolve(ResolveJob J) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= J.n_atoms) return;
     const uint32_t meta = J.meta[t];
     if (meta & kMetaZero) return;
-    uint8_t *dst = J.arc;
-    if (J.dst_off) {
-        dst += J.dst_off[t];
-    } else {
-        const uint64_t a = J.canon_first + t;   // canonical index
-        dst += J.pos[a] + (J.lay.first_in_region(a) ? kL2Bytes : 0ull);
-    }
+    uint8_t *dst = resolve_dst(J, t);
     if (lane == 0) dst[0] = (uint8_t)((meta >> 16) & 0xFFu);
     const uint32_t n = J.len[t] - 6u;   // sums less one
-    if (J.sums && n < kSumsMax) {
-        enc_resolve(J.sums + t * kSums, n, dst + 1, lane);
-    } else {
-        rc_encode_levels_warp<true>(J.ent + t * (uint64_t)VCD_MAX_ENTRIES, meta & 0xFFFFu, lane == 0, J.band_start,
-                                    dst + 1);
+    if (J.sums && n < kSumsMax) enc_resolve(J.sums + t * kSums, n, dst + 1, lane);
+    else if (lane == 0) J.rest[1u + atomicAdd(J.rest, 1u)] = (uint32_t)t;
+}
+
+// The atoms that k_resolve collected, coded from their lists in lockstep, spread
+// evenly over the SM sub-partitions at up to 32 a warp.
+__global__ void __launch_bounds__(128) k_rc_encode_rest(ResolveJob J, uint32_t slots) {
+    __shared__ uint32_t bstart[9];
+    if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, n = J.rest[0];
+    const uint32_t k = (n + 32u * slots - 1u) / (32u * slots), G = k ? (n + k * slots - 1u) / (k * slots) : 1u;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; (uint64_t)w * G < n; w += warps) {
+        const uint32_t i = w * G + lane;
+        const bool on = lane < G && i < n;
+        const uint64_t t = on ? J.rest[1u + i] : 0u;
+        rc_encode_levels_warp<true>(J.ent + t * (uint64_t)VCD_MAX_ENTRIES, on ? J.meta[t] & 0xFFFFu : 0u, on, bstart,
+                                    on ? resolve_dst(J, t) + 1 : nullptr);
     }
 }
 
-void launch_resolve(const ResolveJob &J, cudaStream_t s) {
-    if (J.n_atoms) k_resolve<<<(unsigned)((J.n_atoms + 7) / 8), 256, 0, s>>>(J);
+void launch_resolve(const ResolveJob &J, int num_sms, cudaStream_t s) {
+    if (!J.n_atoms) return;
+    cudaMemsetAsync(J.rest, 0, 4, s);
+    k_resolve<<<(unsigned)((J.n_atoms + 7) / 8), 256, 0, s>>>(J);
+    const uint64_t nb = (J.n_atoms + 3) / 4, cap = 2ull * (uint64_t)num_sms;
+    k_rc_encode_rest<<<(unsigned)(nb < cap ? nb : cap), 128, 0, s>>>(J, 4u * (uint32_t)num_sms);
 }
 
 // consume[a] = (first atom of its region ? L2 block : 0) + payload length

@@ -87,6 +87,7 @@ struct ResolveJob {
     uint32_t band_start[9];
     const uint32_t *len;
     const uint32_t *sums;                // null: code every atom from its list
+    uint32_t *rest;                      // scratch, 1 + n_atoms words: how many atoms are coded from their lists, which
     uint8_t *arc;
     const uint64_t *dst_off;             // optional: per atom (this launch) payload offset in arc
     const uint64_t *pos;                 // else: canonical exclusive scan of consumed bytes
@@ -113,7 +114,7 @@ void enc_tables(EncTables *t, const vcd_tables *vt);   // on the host
 uint64_t size_sets_atoms(int num_sms);
 // atoms that a coder pass runs as groups at most
 uint64_t enc_group_atoms(int num_sms);
-void launch_resolve(const ResolveJob &J, cudaStream_t s);
+void launch_resolve(const ResolveJob &J, int num_sms, cudaStream_t s);
 void launch_consume(const PlaceJob &J, cudaStream_t s);
 void launch_slots(const PlaceJob &J, cudaStream_t s);
 void launch_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, cudaStream_t s);

@@ -81,17 +81,18 @@ static void resolve_range(EncState &S, uint64_t c0, uint64_t n, const uint32_t *
     memcpy(W.band_start, g_dev.band_start, sizeof W.band_start);
     W.len = S.len + c0;
     W.sums = sums;
+    W.rest = meta == S.meta ? S.doubt : S.doubt2;
     W.arc = S.arc;
     W.pos = S.pos;
     W.canon_first = c0;
     W.lay = S.lay;
     const bool prof = vcd_prof_on();
     if (prof) cudaEventRecord(S.c->ev[5], st);
-    launch_resolve(W, st);
+    launch_resolve(W, g_dev.num_sms, st);
     if (prof) {
         cudaEventRecord(S.c->ev[1], st);
         cudaEventSynchronize(S.c->ev[1]);
-        vcd_prof_add("encode_resolve", vcd_elapsed(S.c->ev[5], S.c->ev[1]), 1, 0, 0, n);
+        vcd_prof_add("encode_resolve", vcd_elapsed(S.c->ev[5], S.c->ev[1]), 2, 0, 0, n);
     }
 }
 
@@ -553,12 +554,13 @@ extern "C" int vcd_encode_segments(const vcd_seg *segs, int nseg, const float *q
     cudaStream_t st = c->stream;
     void *p;
     const size_t q_b = ((size_t)nq * sizeof(vcd_quant) + 255) & ~(size_t)255;
-    CK(vcd_scratch(c, VCD_BUF_EMETA, q_b + kWChunk * (4 + 4 + 8 + 1) + 256, &p), "writer metadata");
+    CK(vcd_scratch(c, VCD_BUF_EMETA, q_b + kWChunk * (4 + 4 + 8 + 1 + 4) + 256, &p), "writer metadata");
     vcd_quant *qtab = (vcd_quant *)p;
     uint32_t *dmeta = (uint32_t *)((uint8_t *)p + q_b);
     uint32_t *dlen = dmeta + kWChunk;
     uint64_t *doff = (uint64_t *)(dlen + kWChunk);
-    uint8_t *dqsel = (uint8_t *)(doff + kWChunk);
+    uint32_t *drest = (uint32_t *)(doff + kWChunk);   // 1 + kWChunk
+    uint8_t *dqsel = (uint8_t *)(drest + 1 + kWChunk);
     vcd_quant *qh = (vcd_quant *)malloc((size_t)nq * sizeof(vcd_quant));
     uint64_t *offh = (uint64_t *)malloc(kWChunk * sizeof(uint64_t));
     if (!qh || !offh) { free(qh); free(offh); return 3; }
@@ -628,7 +630,8 @@ extern "C" int vcd_encode_segments(const vcd_seg *segs, int nseg, const float *q
             W.sums = R.sums;
             W.arc = dpack;
             W.dst_off = doff;
-            launch_resolve(W, st);
+            W.rest = drest;
+            launch_resolve(W, g_dev.num_sms, st);
             if (total + bytes > c->wpin_cap) {   // grow the pinned output, keeping what it holds
                 if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
                 size_t want = (total + bytes) + (total + bytes) / 2 + (1 << 20);
