@@ -51,7 +51,8 @@ vc_status vcg_set_batch_shape(int rc_scalar_warps, int transform_threads, int tr
 // the device-output variants (process-wide; results do not depend on it). Up
 // to w warps per SM sub-partition (4 per SM) each atom has a warp running a
 // one-atom decoder, longest payloads first above one per sub-partition, on a
-// copy of its stream in shared memory where the streams fit; above that the
+// copy of its stream in shared memory where the streams fit (by default, up to
+// 28 atoms per SM where they do not); above that the
 // per-lane decoder (every lane of a warp decodes its own atom, atoms in order
 // of payload length; up to 32 atoms per sub-partition the longest four per SM
 // have warps of their own). w = 0: no atom keeps a warp to itself (above one atom

@@ -51,3 +51,10 @@ def test_solo_malformed(vc, gpu):
         finally:
             vc.lib().vcg_set_rc_scalar_warps(-1)
     assert got == [vc.VC_ERR_FORMAT] * 2
+
+
+@pytest.mark.parametrize("rows", [26, 27])   # 4,160 and 4,320 atoms: below and above 28 an SM
+def test_long_streams_change_over(vc, gpu, rows):
+    """Streams too long to be staged: a warp each below the line, a lane each above it."""
+    data, dims = encoded(vc, (32, rows, 5), 0.3)
+    assert (decoded(vc, data, dims, -1, dims[2]) == decoded(vc, data, dims, 64, dims[2])).all()

@@ -343,17 +343,26 @@ static uint32_t stage_bytes_for(uint64_t n, uint32_t max_len, uint32_t sms) {
     return n <= 4ull * sms ? fit : 0u;
 }
 
+constexpr uint32_t kUnstagedPerSm = 28;
+
 // The range decode of every PRESENT box atom:
 //   up to rc_scalar_warps() atoms per SM sub-partition: one atom per warp,
 //     longest payload first above one per sub-partition (the tail is the
-//     shortest atoms), the stream staged in shared memory if all streams fit;
+//     shortest atoms), the stream staged in shared memory if all streams fit
+//     (at the default policy up to kUnstagedPerSm atoms per SM if not: 4,320
+//     atoms at target 10 take 5.75 ms so and 4.39 a lane each, 4,000, which fit,
+//     4.74 and 4.43; of 10 KB streams 4,160 take 9.1 and 8.8, 3,200 8.6 and 8.7);
 //   above: the per-lane decoder over atoms sorted by payload length, the
 //     rc_solo_for() longest on the latency decoder (k_rc_solo, a warp each,
 //     on the second stream of ev, between its fork and join events).
 // Without an order buffer (no-alloc path) the unsorted forms are used.
 static void launch_rc(const DecodeJob &J, int num_sms, cudaStream_t s, const StageEvents *ev) {
-    const uint32_t G = rc_lanes_for(J.n_atoms, (uint32_t)num_sms, rc_scalar_warps());
+    uint32_t G = rc_lanes_for(J.n_atoms, (uint32_t)num_sms, rc_scalar_warps());
     const bool sorted = J.order && J.sort_ctl && rc_sorts(J.n_atoms, (uint32_t)num_sms);
+    const uint32_t stage = G == 1 ? stage_bytes_for(J.n_atoms, J.max_len, (uint32_t)num_sms) : 0u;
+    if (sorted && G == 1 && !stage && rc_scalar_warps() == kRcScalarWarpsDefault &&
+        J.n_atoms > (uint64_t)kUnstagedPerSm * (uint32_t)num_sms)
+        G = 32;
     if (sorted) launch_len_sort(J, s);
     if (G > 1 && sorted) {
         const uint32_t ns = ev && ev->side && ev->fork && ev->join ? rc_solo_for(J.n_atoms, (uint32_t)num_sms) : 0u;
@@ -385,7 +394,6 @@ static void launch_rc(const DecodeJob &J, int num_sms, cudaStream_t s, const Sta
         Jr.order = nullptr;
         Jr.sort_ctl = nullptr;
     }
-    const uint32_t stage = G == 1 ? stage_bytes_for(J.n_atoms, J.max_len, (uint32_t)num_sms) : 0u;
     if (stage) smem_attr((const void *)k_rc_decode, (int)kStageMax);
     k_rc_decode<<<(unsigned)((J.n_atoms + G - 1) / G), 32, stage, s>>>(Jr, G, stage);
 }
