@@ -8,7 +8,9 @@
 //                 shared memory and compacted to (scan position, level) lists
 //   k_rc_encode_groups / k_rc_encode_lanes   range coder (src/vc/vc.c:528-544):
 //                 lengths, and the sums that k_resolve makes payloads
-//                 [dc][bytes] of at their archive offsets (src/vc/vc.c:595-622)
+//                 [dc][bytes] of at their archive offsets (src/vc/vc.c:595-622);
+//                 k_rc_encode_rest codes those too long for their sums there
+//   k_rc_sizes    lengths alone, from the decisions' costs
 //   k_consume / k_slots   canonical layout: bytes consumed per atom in append
 //                 order (an L2 block of 512 KiB at a region's first atom, then the
 //                 payload) and the 16-byte L2 slots (src/vc/vc.c:1082-1159)

@@ -19,7 +19,7 @@ namespace vcg {
 // Words of an atom's slot of sums. Coders check their count every step or pair of
 // rounds (at most 256 decisions of at most 7.05 bits) and at kSumsMax or more go
 // on counting over the slot's last words; such an atom is written by
-// rc_encode_levels_warp instead.
+// k_rc_encode_rest instead.
 constexpr uint32_t kSums = 32768;
 constexpr uint32_t kSumsMax = kSums - 512;
 
@@ -289,9 +289,9 @@ __device__ __forceinline__ void enc_produce(const EncGroup &g, uint32_t slot, co
     }
 }
 
-// The coder warp of a group: lane a codes the group's atom a (list length nnz,
-// last entry `last`) and returns its byte count; its sums go to out (kDigits
-// words of it; past kSumsMax of them the count goes on alone).
+// The coder warp of a group: lane a, where on, codes the group's atom a (eob: its
+// last entry's scan position + 1, or 0) and returns its byte count; its sums go
+// to out, kSums words.
 template <bool WRITE>
 __device__ __forceinline__ uint32_t enc_consume(const EncGroup &g, bool on, uint32_t eob, uint32_t *out,
                                                 uint32_t lane) {
