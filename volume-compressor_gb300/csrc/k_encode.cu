@@ -285,10 +285,14 @@ __global__ void __launch_bounds__(kQuantThreads) k_quant_cached(FwdJob J) {
     __shared__ QuantShared q;
     __shared__ uint32_t wcnt[kQuantThreads / 32];
     const int tid = threadIdx.x;
-    q.load(J.q[0]);
-    __syncthreads();
-    for (uint64_t t = blockIdx.x; t < J.n_atoms; t += gridDim.x) {
-        const uint64_t ca = J.first + t;
+    uint64_t have = ~0ull;
+    for (uint64_t t = blockIdx.x; t < J.n_atoms * J.sets; t += gridDim.x) {
+        const uint64_t set = t / J.n_atoms, ca = J.first + t % J.n_atoms;
+        if (set != have) {   // uniform across the CTA, which is past the previous set's last atom
+            q.load(J.q[set]);
+            have = set;
+            __syncthreads();
+        }
         const uint32_t dcz = J.coef_dc[ca];
         if (dcz & kMetaZero) {
             if (tid == 0) J.meta[t] = kMetaZero;
@@ -527,8 +531,8 @@ void enc_set_smem() {
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s) {
     enc_set_smem();
     if (!J.n_atoms) return;
-    const uint64_t cap = (uint64_t)num_sms * 3;
-    k_quant_cached<<<(unsigned)(J.n_atoms < cap ? J.n_atoms : cap), kQuantThreads, kQuantSmem, s>>>(J);
+    const uint64_t cap = (uint64_t)num_sms * 3, n = J.n_atoms * J.sets;
+    k_quant_cached<<<(unsigned)(n < cap ? n : cap), kQuantThreads, kQuantSmem, s>>>(J);
 }
 
 void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s) {

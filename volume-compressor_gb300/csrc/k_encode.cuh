@@ -44,7 +44,8 @@ struct FwdJob {
     uint32_t dims[8][3];         // nx, ny, nz per LOD
     uint64_t first;              // canonical index of this launch's first atom
     uint64_t n_atoms;
-    const vcd_quant *q;          // per-LOD quantiser constants (device, [lod])
+    const vcd_quant *q;          // per-LOD quantiser constants (device, [lod]); kept transforms: per set
+    uint32_t sets;               // kept transforms: all n_atoms with q[0], then all with q[1], ...
     const uint8_t *qsel;         // optional: per atom (this launch) index into q instead of its LOD
     const uint32_t *place;       // scan position -> index in the transform's tile | quantiser class << 16 (EncTables)
     uint32_t *ent;               // per atom VCD_MAX_ENTRIES slots: scan position | level << 16

@@ -98,7 +98,7 @@ static void resolve_range(EncState &S, uint64_t c0, uint64_t n, const uint32_t *
 
 // forward pass over canonical atoms [c0, c0 + n)
 static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uint32_t *ent, uint32_t *meta,
-                      uint32_t set = 0) {
+                      uint32_t sets = 1) {
     FwdJob F;
     memset(&F, 0, sizeof F);   // fields this pass does not use stay null
     F.lay = S.lay;
@@ -106,7 +106,8 @@ static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uin
     memcpy(F.dims, S.dims, sizeof F.dims);
     F.first = c0;
     F.n_atoms = n;
-    F.q = S.qtab + set;
+    F.q = S.qtab;
+    F.sets = sets;   // more than one only from kept transforms
     F.place = enc_dev()->place;
     F.ent = ent;
     F.meta = meta;
@@ -125,7 +126,7 @@ static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uin
         cudaEventSynchronize(S.c->ev[5]);
         // forward: volume bytes in (the lists it writes are scratch, not counted)
         if (from_cache)   // coefficients in, lists out (scratch, not counted)
-            vcd_prof_add("quant_cached", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * 131072ull, 0, n);
+            vcd_prof_add("quant_cached", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * sets * 131072ull, 0, n * sets);
         else
             vcd_prof_add("fwd_dct_quant", vcd_elapsed(S.c->ev[4], S.c->ev[5]), 1, n * 32768ull, 0, n);
     }
@@ -342,8 +343,7 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         if (pass != RcJob::kDoubt)
             for (uint32_t k = 0; k < sets; ++k) set_q(S, (int)k, m[k].q);
         if (pass == RcJob::kDoubt || sets > 1) {
-            for (uint32_t k = 0; k < sets && pass != RcJob::kDoubt; ++k)   // else the lists are those of the pass before
-                fwd_chunk(S, 0, na0, st, S.ent + k * na0 * VCD_MAX_ENTRIES, S.meta + k * na0, k);
+            if (pass != RcJob::kDoubt) fwd_chunk(S, 0, na0, st, S.ent, S.meta, sets);   // else the lists are at hand
             code_chunk(S, 0, na0, kSizes, st, S.ent, S.meta, nullptr);
         } else {
             run_range(S, 0, na0, kSizes, st, S.ent, S.meta);
