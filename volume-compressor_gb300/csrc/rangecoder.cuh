@@ -563,7 +563,13 @@ struct RcLane {
             }
             if (x == 33u) {   // a prefix longer than any level needs: malformed
                 bad = 1;
-                finish();
+                if (END) {
+                    finish();
+                } else {   // at its end: rounds() takes the other form next, where it finishes
+                    x = 0;
+                    sa = base + kDone;
+                    end = wp;
+                }
             }
         }
         // sign bit and store of a finished level, then the significance of the next position
@@ -608,6 +614,7 @@ struct RcLane {
 #endif
         } else {
             while (o >= 32u) next_word_end();
+            if (bad != 0 && c != kLaneDone) finish();
             if (left == 0 && sa == base) {   // end of the band: a fresh context, or the EOB
                 if (bend == eob) {
                     finish();
@@ -627,7 +634,8 @@ struct RcLane {
 
     // rounds of every lane of the warp until some lane has met an end (whole
     // warp; call until all lanes are done): two at a time, with escape bits in
-    // the second
+    // the second. A lane is done only through the last round here, so that the
+    // loop before it ends when no live lane is left to end it.
     template <int kZ>
     __device__ __forceinline__ void rounds(const uint32_t *bstart) {
         while (!__any_sync(0xFFFFFFFFu, near_end<kZ>())) {
