@@ -2,13 +2,14 @@
 // rangecoder.cuh, RcLane) in the loop that the kernels run it in, decode_lanes of
 // rc_lanes.cuh, with single-lane stand-ins for the CUDA intrinsics (the lanes of
 // a warp are alike). Test infrastructure: every stream of the input file must end
-// within a bounded number of warp votes, with the oracle's status and levels
+// within a bounded number of warp votes, with the oracle's status and levels and
+// without a load of a word that holds no stream byte
 // (tests/test_host_lanes.py writes the file).
 //
 // Input (little-endian): u32 n; per stream: u32 len, u32 bad, u32 nent, then
 // len stream bytes, then nent entries (scan position | level << 16, scan order).
 // Output: one line per form of the loop, "<name> <streams that differ> <streams
-// without an end> <streams>".
+// without an end> <streams with a load outside> <streams>".
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
@@ -21,8 +22,17 @@
 #define __constant__
 
 static inline uint32_t __umulhi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
-static inline uint32_t __ldg(const uint32_t *p) { return *p; }
-static inline uint8_t __ldg(const uint8_t *p) { return *p; }
+// A load of a word without a stream byte (or of a byte outside the stream) is
+// counted and gives ones instead.
+static const uint8_t *g_lo, *g_hi;
+static uint64_t g_outside;
+static inline bool inside(const void *p, size_t n) {
+    const bool in = (const uint8_t *)p < g_hi && (const uint8_t *)p + n > g_lo;
+    g_outside += !in;
+    return in;
+}
+static inline uint32_t __ldg(const uint32_t *p) { return inside(p, 4) ? *p : 0xFFFFFFFFu; }
+static inline uint8_t __ldg(const uint8_t *p) { return inside(p, 1) ? *p : 0xFFu; }
 static inline uint32_t __byte_perm(uint32_t x, uint32_t y, uint32_t s) {
     const uint64_t v = ((uint64_t)y << 32) | x;
     uint32_t r = 0;
@@ -73,6 +83,7 @@ static void band_table(uint32_t *bs) {   // first scan position of each signific
 struct Result {
     bool ended;
     uint32_t bad;
+    uint64_t outside;
     std::vector<uint32_t> ent;
 };
 
@@ -82,7 +93,9 @@ static Result decode(const uint8_t *src, uint32_t len, const uint32_t *bs) {
     std::vector<uint32_t> dst(cap);
     uint32_t S[12];
     RcLane L;
-    g_votes = 0;
+    g_votes = g_outside = 0;
+    g_lo = src;
+    g_hi = src + len;
     bool ended = true;
     try {
         L.init(src, len, true, bs, S, 1, dst.data(), cap);
@@ -90,7 +103,7 @@ static Result decode(const uint8_t *src, uint32_t len, const uint32_t *bs) {
     } catch (const Endless &) {
         ended = false;
     }
-    Result r{ended, L.bad, {}};
+    Result r{ended, L.bad, g_outside, {}};
     for (uint32_t i = 0; i < L.n && i < cap; ++i)
         if (dst[i] >> 16) r.ent.push_back(dst[i]);   // (a raster has no entry for a crafted level 0)
     return r;
@@ -106,7 +119,7 @@ int main(int argc, char **argv) {
     band_table(bs);
     bs[9] = bs[8];
     const char *names[2] = {"dense", "zeros"};
-    int diff[2] = {0, 0}, endless[2] = {0, 0};
+    int diff[2] = {0, 0}, endless[2] = {0, 0}, outside[2] = {0, 0};
     for (uint32_t k = 0; k < n; ++k) {
         uint32_t h[3];
         if (fread(h, 4, 3, f) != 3) return 2;
@@ -124,6 +137,7 @@ int main(int argc, char **argv) {
         const Result r[2] = {decode<0>(src, len, bs), decode<6>(src, len, bs)};
         for (int d = 0; d < 2; ++d) {
             endless[d] += !r[d].ended;
+            outside[d] += r[d].outside != 0;
             const bool same = r[d].ended && (r[d].bad != 0) == (bad != 0) &&
                               (bad || (r[d].ent.size() == nent &&
                                        (!nent || memcmp(r[d].ent.data(), want.data(), 4ull * nent) == 0)));
@@ -132,6 +146,6 @@ int main(int argc, char **argv) {
         delete[] buf;
     }
     fclose(f);
-    for (int d = 0; d < 2; ++d) printf("%s %d %d %u\n", names[d], diff[d], endless[d], n);
+    for (int d = 0; d < 2; ++d) printf("%s %d %d %d %u\n", names[d], diff[d], endless[d], outside[d], n);
     return 0;
 }

@@ -1,6 +1,6 @@
 """The per-lane range decoder in the loop its kernels run (RcLane::rounds, with
 no zeros at once and with six) built for the host (tests/host_lanes.cpp): the
-oracle's status and levels, and an end, on crafted streams whose escape prefix is
+oracle's status and levels, an end and no load of a word outside the stream, on crafted streams whose escape prefix is
 longer than any level needs at every distance from the ends of the band and of
 the stream, on runs of 0xFF, on coded noise, cut and random streams. No GPU needed."""
 import os
@@ -12,7 +12,7 @@ import pytest
 
 from conftest import ROOT
 from rcstream import RangeEncoder
-from test_host_decoders import expected, other_streams
+from test_host_decoders import SANITIZE, expected, other_streams
 
 
 def build(tmp_path_factory, flags, name):
@@ -23,11 +23,16 @@ def build(tmp_path_factory, flags, name):
     return exe, r
 
 
-@pytest.fixture(scope="module")
-def harness(tmp_path_factory):
-    exe, r = build(tmp_path_factory, ["-O2"], "host_lanes")
+@pytest.fixture(scope="module", params=["plain", "sanitized"])
+def harness(tmp_path_factory, request):
+    if request.param == "plain":
+        exe, r = build(tmp_path_factory, ["-O2"], "host_lanes")
+        if r.returncode:
+            pytest.fail(r.stderr[-2000:])
+        return exe
+    exe, r = build(tmp_path_factory, SANITIZE, "host_lanes_san")
     if r.returncode:
-        pytest.fail(r.stderr[-2000:])
+        pytest.skip("no AddressSanitizer / UBSan with this compiler: " + r.stderr[-200:])
     return exe
 
 
@@ -66,7 +71,7 @@ def overlong_streams():
     rng = np.random.default_rng(0x33)
     out = []
     for eob in (1, 5, 12, 200, 4000, 30000):
-        for before in (0, 1, 3, 8, 40):
+        for before in (0, 1, 2, 3, 4, 5, 6, 7, 8, 13, 40):
             if before >= eob:
                 continue
             for ones in (32, 33, 34, 40):
@@ -90,7 +95,7 @@ def run(harness, oracle, streams, tmp_path):
             f.write(ent.astype("<u4").tobytes())
     r = subprocess.run([harness, path], capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stderr[-3000:]
-    return {name: (int(diff), int(endless)) for name, diff, endless, _ in
+    return {name: (int(diff), int(endless), int(outside)) for name, diff, endless, outside, _ in
             (line.split() for line in r.stdout.strip().splitlines())}
 
 
@@ -98,8 +103,8 @@ def test_overlong_prefix_ends(harness, oracle, tmp_path):
     streams = overlong_streams()
     bad = [expected(oracle, s)[0] for s in streams]
     assert sum(bad) > len(streams) // 3 and sum(bad) < len(streams)
-    assert run(harness, oracle, streams, tmp_path) == {"dense": (0, 0), "zeros": (0, 0)}
+    assert run(harness, oracle, streams, tmp_path) == {"dense": (0, 0, 0), "zeros": (0, 0, 0)}
 
 
 def test_noise_cut_and_random_streams(harness, oracle, tmp_path):
-    assert run(harness, oracle, other_streams(oracle), tmp_path) == {"dense": (0, 0), "zeros": (0, 0)}
+    assert run(harness, oracle, other_streams(oracle), tmp_path) == {"dense": (0, 0, 0), "zeros": (0, 0, 0)}

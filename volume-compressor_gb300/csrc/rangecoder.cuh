@@ -388,7 +388,8 @@ struct RcLane {
         wp += 4;
         return v;
     }
-    __device__ __forceinline__ void finish() {   // nothing of the lane is near an end any more
+    // nothing of the lane is near an end any more; only where no stream word is due (o < 32)
+    __device__ __forceinline__ void finish() {
         sa = base + kDone;
         left = 0x40000000u;
         end = wp + 64;
@@ -562,14 +563,10 @@ struct RcLane {
                 mag = on ? mn : mag;
             }
             if (x == 33u) {   // a prefix longer than any level needs: malformed
-                bad = 1;
-                if (END) {
-                    finish();
-                } else {   // at its end: rounds() takes the other form next, where it finishes
-                    x = 0;
-                    sa = base + kDone;
-                    end = wp;
-                }
+                bad = 1;      // at its end, without a part in what follows; END finishes the lane
+                x = 0;
+                sa = base + kDone;
+                end = wp;
             }
         }
         // sign bit and store of a finished level, then the significance of the next position
@@ -614,7 +611,7 @@ struct RcLane {
 #endif
         } else {
             while (o >= 32u) next_word_end();
-            if (bad != 0 && c != kLaneDone) finish();
+            if (sa == base + kDone) finish();   // (after the last load: finish() lifts the guard of load_word())
             if (left == 0 && sa == base) {   // end of the band: a fresh context, or the EOB
                 if (bend == eob) {
                     finish();
