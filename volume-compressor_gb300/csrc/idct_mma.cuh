@@ -31,6 +31,7 @@
 #include <stdint.h>
 
 #include "dct32.cuh"
+#include "feed_extent.cuh"
 #include "idct_tile.cuh"
 
 namespace vcg {
@@ -210,8 +211,7 @@ struct MmaShared {
     MmaAtom atom[kMmaAtoms];
     uint32_t count[kMmaChunks];   // entries of the chunk | kMmaLast
     uint32_t tmem;             // TMEM base
-    float norm[kMmaFeeders / 32];
-    uint32_t far[kMmaFeeders / 32];
+    FeedExtent<kMmaFeeders / 32> extent;
     int2 dq[VCD_NCLASS];       // step, bias + 128 of the feeders' LOD
 };
 constexpr uint32_t kMmaLast = 1u << 30;
@@ -339,15 +339,13 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
 #pragma unroll
                 for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
                 const uint32_t fw = __reduce_max_sync(0xFFFFFFFFu, far);
-                if (lane == 0) {
-                    M.norm[warp] = s;
-                    M.far[warp] = fw;
-                }
+                if (lane == 0) M.extent.put(i, warp, s, fw);
                 mma_sync_feeders();
                 if (tid == 0) {
-                    s = M.norm[0] + M.norm[1] + M.norm[2];
+                    uint32_t f;
+                    M.extent.take(i, s, f);
                     a.fits = s <= kMmaNorm * kMmaNorm;   // (NaN or infinite: no)
-                    a.tiles = max(max(M.far[0], M.far[1]), M.far[2]) / kMmaTile + 1u;
+                    a.tiles = f / kMmaTile + 1u;
                 }
             }
             if (tid == 0) M.count[slot] = m | (last ? kMmaLast : 0u);
