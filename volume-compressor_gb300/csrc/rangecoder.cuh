@@ -609,12 +609,10 @@ struct RcLane {
 #endif
         } else {
             while (o >= 32u) next_word_end();
-            if (x == 33u) {   // after the round's last load: finish() lifts the guard of load_word()
-                x = 0;
-                finish();
-            }
-            if (left == 0 && sa == base) {   // end of the band: a fresh context, or the EOB
-                if (bend == eob) {
+            const bool malformed = x == 33u;
+            if (malformed || (left == 0 && sa == base)) {   // or the end of the band: a fresh context, or the EOB
+                if (malformed || bend == eob) {   // (past the round's last load: finish() lifts the guard of load_word())
+                    x = 0;
                     finish();
                 } else {
                     ++bi;
