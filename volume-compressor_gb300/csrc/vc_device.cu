@@ -881,12 +881,12 @@ static int decode_job(vcd_ctx *c, const uint8_t *arc, const vcd_atom *atoms, uin
             cudaGetLastError();
             return vcd_status_of(e);
         }
-        if ((e = cudaMemcpyAsync(ctl_h, p_ctl, 16, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess) {
-            vcd_set_error("decode status copy", e);
-            return vcd_status_of(e);
-        }
     }
-    if (piped) cudaMemcpyAsync(ctl_h, p_ctl, 16, cudaMemcpyDeviceToHost, c->stream);   // as the transform left it
+    // the control words as the transform left them
+    if ((e = cudaMemcpyAsync(ctl_h, p_ctl, 16, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess) {
+        vcd_set_error("decode status copy", e);
+        return vcd_status_of(e);
+    }
     if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess || (piped && (e = cudaStreamSynchronize(c->copy_stream)) != cudaSuccess) ||
         (e = cudaGetLastError()) != cudaSuccess) {
         vcd_set_error("decode kernels", e);
