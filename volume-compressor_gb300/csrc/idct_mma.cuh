@@ -46,9 +46,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)_
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-// Waits until the phase of parity `parity` is complete; false after about a second.
+// Waits until the phase of parity `parity` is complete; false after a quarter of a
+// second (a try gives up after 4 us on GB300, whatever the hint; TIMES: so many
+// quarters). What the CTA's roles wait for takes some 10 us an atom.
+#ifndef VCG_WAIT_TRIES
+#define VCG_WAIT_TRIES (1u << 16)
+#endif
+template <uint32_t TIMES = 1>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < (1u << 16); ++i) {
+    for (uint32_t i = 0; i < TIMES * VCG_WAIT_TRIES; ++i) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 0x4000;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}"
@@ -208,9 +214,12 @@ struct MmaShared {
     uint64_t second[8];        // a tile's second operand is written: per warp of its group
     uint64_t third;            // the third operand is written: per warp of the 16
     uint64_t full[kMmaChunks], empty[kMmaChunks];
+    uint64_t drained;          // the issuing thread is done with the tensor cores
     MmaAtom atom[kMmaAtoms];
     uint32_t count[kMmaChunks];   // entries of the chunk | kMmaLast
     uint32_t tmem;             // TMEM base
+    uint32_t gave_up;          // a wait of the 16 warps ran out: set before an arrival at scattered, read after them all
+    uint32_t starved;          // a wait of the feeders did
     FeedExtent<kMmaFeeders / 32> extent;
     int2 dq[VCD_NCLASS];       // step, bias + 128 of the feeders' LOD
 };
@@ -218,18 +227,20 @@ constexpr uint32_t kMmaLast = 1u << 30;
 
 __device__ __forceinline__ void mma_sync16() { asm volatile("bar.sync %0, %1;" ::"n"(kMmaBar), "n"(kMmaThreads) : "memory"); }
 __device__ __forceinline__ void mma_sync_feeders() { asm volatile("bar.sync 6, %0;" ::"n"(kMmaFeeders) : "memory"); }
-// mma_sync16; true on every thread if v is true on one
-__device__ __forceinline__ bool mma_sync16_or(bool v) {
+// A barrier of NT threads; true on every thread if v is true on one
+template <int BAR, int NT>
+__device__ __forceinline__ bool mma_sync_or(bool v) {
     uint32_t r;
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred p, %2, %3, p;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(r)
-                 : "r"((uint32_t)v), "n"(kMmaBar), "n"(kMmaThreads)
+                 : "r"((uint32_t)v), "n"(BAR), "n"(NT)
                  : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void mma_arrive(uint64_t &bar) {   // one arrival per warp
+__device__ __forceinline__ bool mma_sync16_or(bool v) { return mma_sync_or<kMmaBar, kMmaThreads>(v); }
+__device__ __forceinline__ void mma_arrive(uint64_t &bar, bool on = true) {   // one arrival per warp, if on its first lane
     __syncwarp();
-    if ((threadIdx.x & 31) == 0)
+    if ((threadIdx.x & 31) == 0 && on)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar)) : "memory");
 }
 
@@ -240,6 +251,8 @@ __device__ __forceinline__ void mma_setup(MmaShared &M, uint8_t *B) {
         for (int i = 0; i < 24; ++i) mbar_init(smem_u32(&M.bar[i]), 1);
         mbar_init(smem_u32(&M.scattered), kMmaThreads / 32);
         mbar_init(smem_u32(&M.third), kMmaThreads / 32);
+        mbar_init(smem_u32(&M.drained), 1);
+        M.gave_up = M.starved = 0;
         for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&M.stored[i]), 4);
         for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&M.second[i]), 4);
         for (uint32_t i = 0; i < kMmaChunks; ++i) {
@@ -266,12 +279,15 @@ __device__ __forceinline__ void mma_release(MmaShared &M) {
 // after the last one (called by one warp, 32 atoms at once, so that their table
 // entries, counts and offsets load together); dq: the LODs' tables; place: see
 // vcd_tables.
+// A thread whose wait for a free chunk ran out writes no chunk any more but meets
+// the others at every barrier, until they all return before the next 32 atoms.
 template <class Describe>
 __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_dq *dq, const uint32_t *place,
                                          Describe &&describe) {
     const int tid = threadIdx.x - kMmaFeed, lane = tid & 31, warp = tid >> 5;
     constexpr int kB = kMmaChunk / kMmaFeeders;   // a chunk's list loads, then its lookups, in flight together
     uint32_t c = 0;        // chunks handed over
+    bool ok = true;
     int lod = -1;
     uint32_t w[kB];        // the list of the chunk in hand: loaded while the one before is worked on
     auto load = [&](const uint32_t *src, uint32_t m) {
@@ -287,7 +303,7 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
                 a.more = describe(i + lane, a);
                 M.atom[(i + lane) % kMmaAtoms] = a;
             }
-            mma_sync_feeders();
+            if (mma_sync_or<6, kMmaFeeders>(!ok)) return;
         }
         MmaAtom &a = M.atom[i % kMmaAtoms];
         const bool more = a.more;
@@ -319,7 +335,10 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
                 const MmaAtom &b = M.atom[(i + 1) % kMmaAtoms];
                 load(b.src, entries(b));
             }
-            if (use && !mbar_wait(smem_u32(&M.empty[slot]), (use + 1u) & 1u)) return;   // (the 16 warps have given up)
+            if (use && ok && !mbar_wait(smem_u32(&M.empty[slot]), (use + 1u) & 1u)) {
+                ok = false;
+                M.starved = 1;
+            }
             uint2 *E = reinterpret_cast<uint2 *>(ring) + slot * kMmaChunk;
 #pragma unroll
             for (int j = 0; j < kB; ++j)
@@ -332,7 +351,7 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
                     norm = __fmaf_rn(f, f, norm);
                     const uint32_t at = r[j] & 0x1FFFFu;
                     far = max(far, at);
-                    E[j * kMmaFeeders + tid] = make_uint2(at, mma_pieces(kMagicBits + (uint32_t)v));
+                    if (ok) E[j * kMmaFeeders + tid] = make_uint2(at, mma_pieces(kMagicBits + (uint32_t)v));
                 }
             if (last && more) {   // the atom's norm and extent along kz (4,096 bytes each)
                 float s = norm;
@@ -348,8 +367,8 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
                     a.tiles = f / kMmaTile + 1u;
                 }
             }
-            if (tid == 0) M.count[slot] = m | (last ? kMmaLast : 0u);
-            mma_arrive(M.full[slot]);
+            if (tid == 0 && ok) M.count[slot] = m | (last ? kMmaLast : 0u);
+            mma_arrive(M.full[slot], ok);
             ++c;
             if (last) break;
         }
@@ -357,13 +376,13 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
     }
 }
 
-// The issuing thread.
-__device__ __forceinline__ void mma_issue(MmaShared &M, uint32_t a, uint32_t b) {
+// The issuing thread, up to the last atom or a wait that ran out.
+__device__ __forceinline__ void mma_issue_atoms(MmaShared &M, uint32_t a, uint32_t b) {
     const uint32_t bar = smem_u32(M.bar), second = smem_u32(M.second), stored = smem_u32(M.stored);
     constexpr uint32_t tile = kMmaTile >> 4;
     uint32_t parity = 0;
     for (uint32_t i = 0;; ++i) {
-        if (!mbar_wait(smem_u32(&M.scattered), i & 1u)) return;
+        if (!mbar_wait(smem_u32(&M.scattered), i & 1u) || M.gave_up) return;
         const MmaAtom &at = M.atom[i % kMmaAtoms];
         if (!at.more) return;
         const bool tensor = at.tensor && at.fits;
@@ -395,6 +414,13 @@ __device__ __forceinline__ void mma_issue(MmaShared &M, uint32_t a, uint32_t b) 
     }
 }
 
+// The issuing thread; when it returns, nothing is in flight any more (TMEM may be freed).
+__device__ __forceinline__ void mma_issue(MmaShared &M, uint32_t a, uint32_t b) {
+    mma_issue_atoms(M, a, b);
+    tc_commit(smem_u32(&M.drained));
+    mbar_wait(smem_u32(&M.drained), 0u);
+}
+
 __device__ __forceinline__ void mma_clear(uint8_t *A) {
     uint4 *A4 = reinterpret_cast<uint4 *>(A) + threadIdx.x;
 #pragma unroll
@@ -404,7 +430,13 @@ __device__ __forceinline__ void mma_clear(uint8_t *A) {
 // The 16 warps: every atom the feeders describe. out(a, y, x, z, o) receives a
 // (y, x) line's outputs z .. z + 15 along z (z = 0, 16) as magic numbers, x =
 // the lane; other(a, A) transforms an atom that is not for the tensor cores, with
-// A (kMmaA bytes at least; left as it is) at hand. False when a wait ran out.
+// A (kMmaA bytes at least; left as it is) at hand. False, on every thread, when a
+// wait ran out.
+//
+// No warp leaves alone, so that none is missed at a barrier: a warp whose wait
+// ran out goes on to the next scatter, says so before its arrival there, and all
+// of them return once they have all arrived. That last wait cannot run out: each
+// warp's scatter is at most 23 waits.
 //
 // The passes of an atom follow one another through the same operand space and
 // sums, so an atom alone leaves the tensor cores idle in between. Its last
@@ -437,7 +469,7 @@ __device__ __forceinline__ bool mma_atoms(uint8_t *A, MmaShared &M, const uint8_
         uint32_t flags;
         do {   // scatter
             const uint32_t slot = c % kMmaChunks;
-            ok &= mbar_wait(smem_u32(&M.full[slot]), (c / kMmaChunks) & 1u);
+            ok = __all_sync(0xFFFFFFFFu, ok && mbar_wait(smem_u32(&M.full[slot]), (c / kMmaChunks) & 1u));
             flags = ok ? M.count[slot] : kMmaLast;
             const uint32_t m = flags & 0xFFFFu;
             const uint2 *E = reinterpret_cast<const uint2 *>(ring) + slot * kMmaChunk;
@@ -448,11 +480,12 @@ __device__ __forceinline__ bool mma_atoms(uint8_t *A, MmaShared &M, const uint8_
                     *reinterpret_cast<uint16_t *>(A + e.x) = (uint16_t)e.y;
                     *reinterpret_cast<uint16_t *>(A + (e.x ^ 64u)) = (uint16_t)(e.y >> 16);   // l: the row's other half
                 }
-            mma_arrive(M.empty[slot]);
+            mma_arrive(M.empty[slot], ok);
             ++c;
         } while (!(flags & kMmaLast));
         const MmaAtom &at = M.atom[i % kMmaAtoms];
         fence_async_smem();
+        if (!ok) M.gave_up = 1;
         mma_arrive(M.scattered);
         if (pending) {   // the atom before: its last outputs
             const MmaAtom &b = M.atom[(i + kMmaAtoms - 1u) % kMmaAtoms];
@@ -463,7 +496,8 @@ __device__ __forceinline__ bool mma_atoms(uint8_t *A, MmaShared &M, const uint8_
         } else {
             mma_arrive(M.stored[group]);
         }
-        if (!at.more) return !mma_sync16_or(!ok);
+        if (!mbar_wait<32>(smem_u32(&M.scattered), i & 1u) || M.gave_up) return false;
+        if (!at.more) return true;
         if (!(at.tensor && at.fits)) {
             mma_sync16();
             other(at, A);

@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(kMmaCta, 1) k_idct(DecodeJob J) {
         if (!ok) atomicExch(J.fail, 1u);   // a wait ran out: the call fails
     }
     mma_release(M);
+    if (tid == 0 && M.starved) atomicExch(J.fail, 1u);
 }
 
 void launch_scan_u64(uint64_t *v, uint64_t n, uint64_t base, uint64_t *total, cudaStream_t s) {
