@@ -461,29 +461,31 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveJob J) {
 }
 
 // The atoms that k_resolve collected, coded from their lists in lockstep, spread
-// evenly over the SM sub-partitions at up to 32 a warp.
+// evenly over the SM sub-partitions (slots) at up to 32 a warp; every atom has its
+// warp, a loop over them would spill.
 __global__ void __launch_bounds__(128) k_rc_encode_rest(ResolveJob J, uint32_t slots) {
     __shared__ uint32_t bstart[9];
     if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, n = J.rest[0];
     const uint32_t k = (n + 32u * slots - 1u) / (32u * slots), G = k ? (n + k * slots - 1u) / (k * slots) : 1u;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; (uint64_t)w * G < n; w += warps) {
-        const uint32_t i = w * G + lane;
-        const bool on = lane < G && i < n;
-        const uint64_t t = on ? J.rest[1u + i] : 0u;
-        rc_encode_levels_warp<true>(J.ent + t * (uint64_t)VCD_MAX_ENTRIES, on ? J.meta[t] & 0xFFFFu : 0u, on, bstart,
-                                    on ? resolve_dst(J, t) + 1 : nullptr);
-    }
+    const uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G;
+    if (i0 >= n) return;
+    const uint32_t i = (uint32_t)i0 + lane;
+    const bool on = lane < G && i < n;
+    const uint64_t t = on ? J.rest[1u + i] : 0u;
+    rc_encode_levels_warp<true>(J.ent + t * (uint64_t)VCD_MAX_ENTRIES, on ? J.meta[t] & 0xFFFFu : 0u, on, bstart,
+                                on ? resolve_dst(J, t) + 1 : nullptr);
 }
 
 void launch_resolve(const ResolveJob &J, int num_sms, cudaStream_t s) {
     if (!J.n_atoms) return;
     cudaMemsetAsync(J.rest, 0, 4, s);
     k_resolve<<<(unsigned)((J.n_atoms + 7) / 8), 256, 0, s>>>(J);
-    const uint64_t nb = (J.n_atoms + 3) / 4, cap = 2ull * (uint64_t)num_sms;
-    k_rc_encode_rest<<<(unsigned)(nb < cap ? nb : cap), 128, 0, s>>>(J, 4u * (uint32_t)num_sms);
+    // the most warps that a rest of 1..n_atoms atoms has
+    const uint64_t slots = 4ull * (uint64_t)num_sms, k = (J.n_atoms + 32 * slots - 1) / (32 * slots);
+    const uint64_t warps = J.n_atoms < k * slots ? J.n_atoms : k * slots;
+    k_rc_encode_rest<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(J, (uint32_t)slots);
 }
 
 // consume[a] = (first atom of its region ? L2 block : 0) + payload length
