@@ -8,8 +8,9 @@
 //                 shared memory and compacted to (scan position, level) lists
 //   k_rc_encode_groups / k_rc_encode_lanes   range coder (src/vc/vc.c:528-544):
 //                 lengths, and the sums that k_resolve makes payloads
-//                 [dc][bytes] of at their archive offsets (src/vc/vc.c:595-622);
-//                 k_rc_encode_rest codes those too long for their sums there
+//                 [dc][bytes] of at their archive offsets (src/vc/vc.c:595-622)
+//   k_long / k_rc_encode_long   atoms too long for their sums: the bytes, which
+//                 k_resolve copies; k_rc_encode_rest: without room for sums
 //   k_rc_sizes    lengths alone, from the decisions' costs
 //   k_consume / k_slots   canonical layout: bytes consumed per atom in append
 //                 order (an L2 block of 512 KiB at a region's first atom, then the
@@ -308,13 +309,21 @@ __global__ void __launch_bounds__(kQuantThreads) k_quant_cached(FwdJob J) {
 
 constexpr size_t size_smem(int A) { return sizeof(EncCosts) + 8 * (size_t)A * kRingPitch * 4; }
 
-// Atom t's list, or none; whether it is present (its dc is coded).
-__device__ __forceinline__ bool enc_atom(const RcJob &J, uint64_t t, const uint32_t *&ent, uint32_t &nnz) {
+// Atom t's list, or none; whether it is present (its dc is coded) and not among
+// those marked `without`.
+__device__ __forceinline__ bool enc_atom(const RcJob &J, uint64_t t, const uint32_t *&ent, uint32_t &nnz,
+                                         uint32_t without = 0u) {
     const uint32_t meta = t < J.n_atoms ? J.meta[t] : kMetaZero;
-    const bool on = !(meta & kMetaZero);
+    const bool on = !(meta & (kMetaZero | without));
     nnz = on ? meta & 0xFFFFu : 0u;
     ent = J.ent + (on ? t : 0) * (uint64_t)VCD_MAX_ENTRIES;
     return on;
+}
+
+// Atom t is left to k_rc_encode_long.
+__device__ __forceinline__ void mark_long(const RcJob &J, uint64_t t) {
+    J.meta[t] |= kMetaLong;
+    J.longs[1u + atomicAdd(J.longs, 1u)] = (uint32_t)t;
 }
 
 // Few atoms: kEncGroups groups of G atoms per CTA. Warps 0..3 code, the warps
@@ -337,13 +346,14 @@ __global__ void __launch_bounds__(32 * kEncGroups * enc_group_warps(kGroupMax)) 
         t = t >= n ? J.n_atoms : SUMS ? t : J.doubt[1u + t];
         const uint32_t *ent;
         uint32_t nnz;
-        const bool on = enc_atom(J, t, ent, nnz);
+        const bool on = enc_atom(J, t, ent, nnz, SUMS ? kMetaLong : 0u);
         if (w == 0u) {
             const uint32_t eob = nnz ? (ent[nnz - 1u] & 0xFFFFu) + 1u : 0u;
             const uint32_t k = enc_consume<SUMS>(g, on, eob, SUMS ? J.sums + (on ? t : 0) * kSums : nullptr, lane);
             if (t < J.n_atoms) {
                 if (!SUMS && on) atomicAdd(J.totals + 3 * (t / J.per), (unsigned long long)(k + 1u - J.len[t]));
                 J.len[t] = on ? k + 1u : 0u;
+                if (SUMS && on && k >= kSumsMax + 5u) mark_long(J, t);
             }
         } else {
             const bool split = enc_group_split(G);
@@ -433,9 +443,10 @@ __global__ void __launch_bounds__(32 * kLanesWarps) k_rc_encode_lanes(RcJob J, u
     const uint64_t t = lane < G ? ((uint64_t)blockIdx.x * kLanesWarps + warp) * G + lane : J.n_atoms;
     const uint32_t *ent;
     uint32_t nnz;
-    const bool on = enc_atom(J, t, ent, nnz);
+    const bool on = enc_atom(J, t, ent, nnz, kMetaLong);
     const uint32_t n = enc_lanes<4, 3, 2>(on, ent, nnz, bstart, J.sums + (on ? t : 0) * kSums, mem[warp], lane);
     if (t < J.n_atoms) J.len[t] = on ? n + 1u : 0u;
+    if (on && n >= kSumsMax + 5u) mark_long(J, t);
 }
 
 // Where the payload of atom t goes.
@@ -445,8 +456,12 @@ __device__ __forceinline__ uint8_t *resolve_dst(const ResolveJob &J, uint64_t t)
     return J.arc + J.pos[a] + (J.lay.first_in_region(a) ? kL2Bytes : 0ull);
 }
 
-// A warp per atom: [dc] and the coder bytes; atoms with more sums than their slot
-// holds are collected for k_rc_encode_rest.
+// Bytes that a slot of sums holds.
+constexpr uint32_t kSlotBytes = kSums * 4u;
+
+// A warp per atom: [dc] and the coder bytes, from its sums or, if it is marked
+// long, from its slot; without slots, or past one, it is collected for
+// k_rc_encode_rest.
 __global__ void __launch_bounds__(256) k_resolve(ResolveJob J) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -456,36 +471,97 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveJob J) {
     uint8_t *dst = resolve_dst(J, t);
     if (lane == 0) dst[0] = (uint8_t)((meta >> 16) & 0xFFu);
     const uint32_t n = J.len[t] - 6u;   // sums less one
-    if (J.sums && n < kSumsMax) enc_resolve(J.sums + t * kSums, n, dst + 1, lane);
-    else if (lane == 0) J.rest[1u + atomicAdd(J.rest, 1u)] = (uint32_t)t;
+    if (J.sums && !(meta & kMetaLong)) {
+        enc_resolve(J.sums + t * kSums, n, dst + 1, lane);
+    } else if (J.sums && n + 5u <= kSlotBytes) {
+        for (uint32_t i = lane; i < (n + 8u) / 4u; i += 32u) {
+            const uint32_t w = J.sums[t * kSums + i];
+            for (uint32_t k = 0; k < 4u && 4u * i + k < n + 5u; ++k) dst[1u + 4u * i + k] = (uint8_t)(w >> (8u * k));
+        }
+    } else if (lane == 0) {
+        J.rest[1u + atomicAdd(J.rest, 1u)] = (uint32_t)t;
+    }
 }
 
-// The atoms that k_resolve collected, coded from their lists in lockstep, spread
-// evenly over the SM sub-partitions (slots) at up to 32 a warp; every atom has its
-// warp, a loop over them would spill.
-__global__ void __launch_bounds__(128) k_rc_encode_rest(ResolveJob J, uint32_t slots) {
-    __shared__ uint32_t bstart[9];
-    if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u, n = J.rest[0];
+// The calling warp's atoms of a list (how many, which) coded in lockstep from
+// their lists, the atoms spread evenly over the SM sub-partitions (slots) at up to
+// 32 a warp; every atom has its warp, a loop over them would spill. dst(t): where
+// its bytes go; done(t, n): called with their count.
+template <class Dst, class Done>
+__device__ __forceinline__ void code_listed(const uint32_t *list, uint32_t slots, const uint32_t *ent,
+                                            const uint32_t *meta, const uint32_t *bstart, uint32_t cap, Dst &&dst,
+                                            Done &&done) {
+    const uint32_t lane = threadIdx.x & 31u, n = list[0];
     const uint32_t k = (n + 32u * slots - 1u) / (32u * slots), G = k ? (n + k * slots - 1u) / (k * slots) : 1u;
     const uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G;
     if (i0 >= n) return;
     const uint32_t i = (uint32_t)i0 + lane;
     const bool on = lane < G && i < n;
-    const uint64_t t = on ? J.rest[1u + i] : 0u;
-    rc_encode_levels_warp<true>(J.ent + t * (uint64_t)VCD_MAX_ENTRIES, on ? J.meta[t] & 0xFFFFu : 0u, on, bstart,
-                                on ? resolve_dst(J, t) + 1 : nullptr);
+    const uint64_t t = on ? list[1u + i] : 0u;
+    const uint32_t bytes = rc_encode_levels_warp<true>(ent + t * (uint64_t)VCD_MAX_ENTRIES, on ? meta[t] & 0xFFFFu : 0u,
+                                                       on, bstart, on ? dst(t) : nullptr, cap);
+    if (on) done(t, bytes);
+}
+
+// the CTAs of 128 threads that code a list of up to n_atoms
+static unsigned listed_ctas(uint64_t n_atoms, uint64_t slots) {
+    const uint64_t k = (n_atoms + 32 * slots - 1) / (32 * slots), warps = n_atoms < k * slots ? n_atoms : k * slots;
+    return (unsigned)((warps + 3) / 4);
+}
+
+__global__ void __launch_bounds__(128) k_rc_encode_rest(ResolveJob J, uint32_t slots) {
+    __shared__ uint32_t bstart[9];
+    if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
+    __syncthreads();
+    code_listed(J.rest, slots, J.ent, J.meta, bstart, 0xFFFFFFFFu, [&](uint64_t t) { return resolve_dst(J, t) + 1; },
+                [](uint64_t, uint32_t) {});
 }
 
 void launch_resolve(const ResolveJob &J, int num_sms, cudaStream_t s) {
     if (!J.n_atoms) return;
     cudaMemsetAsync(J.rest, 0, 4, s);
     k_resolve<<<(unsigned)((J.n_atoms + 7) / 8), 256, 0, s>>>(J);
-    // the most warps that a rest of 1..n_atoms atoms has
-    const uint64_t slots = 4ull * (uint64_t)num_sms, k = (J.n_atoms + 32 * slots - 1) / (32 * slots);
-    const uint64_t warps = J.n_atoms < k * slots ? J.n_atoms : k * slots;
-    k_rc_encode_rest<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(J, (uint32_t)slots);
+    const uint32_t slots = 4u * (uint32_t)num_sms;
+    k_rc_encode_rest<<<listed_ctas(J.n_atoms, slots), 128, 0, s>>>(J, slots);
+}
+
+// Atoms with more sums than their slot holds (white noise at the finest
+// quantisers) are coded from their lists after the others, their bytes into the
+// slot. The coder marks them when it is done. Where there are more than its groups
+// take, its own pass would cost nearly as much, so an atom is marked before it, and
+// left out, if the bypass decisions of its list's escapes and signs alone, a bit
+// each, tell it: a warp per atom; only a list that can be long is read.
+constexpr uint32_t kLongBits = 8u * kSumsMax;
+__global__ void __launch_bounds__(256) k_long(RcJob J) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (t >= J.n_atoms) return;
+    const uint32_t meta = J.meta[t], nnz = meta & 0xFFFFu;
+    if (meta & kMetaZero || nnz < kLongBits / 32u) return;   // an entry has at most 32
+    const uint32_t *ent = J.ent + t * (uint64_t)VCD_MAX_ENTRIES;
+    uint32_t sum = 0;
+    for (uint32_t i = lane; i < nnz; i += 32u) {
+        const int32_t lv = (int32_t)__ldg(ent + i) >> 16;
+        uint32_t bits;
+        sum += enc_tail((uint32_t)(lv < 0 ? -lv : lv), false, &bits);
+    }
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+    if (lane == 0 && sum >= kLongBits) mark_long(J, t);
+}
+
+__global__ void __launch_bounds__(128) k_rc_encode_long(RcJob J, uint32_t slots) {
+    __shared__ uint32_t bstart[9];
+    if (threadIdx.x < 9) bstart[threadIdx.x] = J.band_start[threadIdx.x];
+    __syncthreads();
+    code_listed(J.longs, slots, J.ent, J.meta, bstart, kSlotBytes,
+                [&](uint64_t t) { return reinterpret_cast<uint8_t *>(J.sums + t * kSums); },
+                [&](uint64_t t, uint32_t n) { J.len[t] = n + 1u; });
+}
+
+void launch_rc_long(const RcJob &J, int num_sms, cudaStream_t s) {
+    if (!J.n_atoms) return;
+    const uint32_t slots = 4u * (uint32_t)num_sms;
+    k_rc_encode_long<<<listed_ctas(J.n_atoms, slots), 128, 0, s>>>(J, slots);
 }
 
 // consume[a] = (first atom of its region ? L2 block : 0) + payload length
@@ -517,8 +593,9 @@ __global__ void k_slots(PlaceJob J) {
     for (int i = 0; i < 16; ++i) slot[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
 }
 
-__global__ void k_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc) {
+__global__ void k_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, uint32_t *zero) {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) *zero = 0;
     if (t < n) dc[t] = (meta[t] & kMetaZero) ? 0 : (uint8_t)(meta[t] >> 16);
 }
 
@@ -610,6 +687,7 @@ void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s) {
         k_rc_encode_groups<true><<<nb, nt, kEncGroups * enc_group_bytes(G), s>>>(J, G);
         return;
     }
+    k_long<<<(unsigned)((J.n_atoms + 7) / 8), 256, 0, s>>>(J);
     const uint64_t k = (J.n_atoms + 32 * slots - 1) / (32 * slots);
     const uint32_t G = (uint32_t)((J.n_atoms + k * slots - 1) / (k * slots));
     const uint64_t warps = (J.n_atoms + G - 1) / G;
@@ -624,8 +702,8 @@ void launch_slots(const PlaceJob &J, cudaStream_t s) {
     k_slots<<<(unsigned)((J.n_total + 255) / 256), 256, 0, s>>>(J);
 }
 
-void launch_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, cudaStream_t s) {
-    k_gather_dc<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(meta, n, dc);
+void launch_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, uint32_t *zero, cudaStream_t s) {
+    k_gather_dc<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(meta, n, dc, zero);
 }
 
 }  // namespace vcg

@@ -9,7 +9,8 @@ namespace vcg {
 
 constexpr uint64_t kL2Bytes = 32768ull * 16ull;   // one region's slot block
 constexpr uint32_t kMetaZero = 1u << 31;           // meta: all-zero atom
-// meta = nnz (bits 0-15, up to 32768) | dc << 16 | kMetaZero
+constexpr uint32_t kMetaLong = 1u << 30;           // more coder bytes than a slot of sums holds (launch_rc_encode)
+// meta = nnz (bits 0-15, up to 32768) | dc << 16 | kMetaLong | kMetaZero
 
 // Canonical append order: LOD-major, atoms in raster (z, y, x) order.
 struct Layout {
@@ -65,11 +66,12 @@ struct EncCosts;
 // Coder pass over the lists of n_atoms atoms: lengths, and sums or totals.
 struct RcJob {
     uint64_t n_atoms;
-    const uint32_t *meta;
+    uint32_t *meta;
     const uint32_t *ent;
     uint32_t band_start[9];
     uint32_t *len;                       // payload bytes per atom ([dc] + coder bytes; 0 = zero atom)
     uint32_t *sums;                      // kSums words per atom, what k_resolve makes the bytes of; null: lengths alone
+    uint32_t *longs;                     // with sums: 1 + n_atoms words: how many atoms are kMetaLong (0 before), which
     // lengths alone
     const EncCosts *costs;
     uint32_t *doubt;                     // scratch, 1 + n_atoms words: how many atoms only the coder can size, which
@@ -84,7 +86,7 @@ struct RcJob {
 struct ResolveJob {
     uint64_t n_atoms;
     const uint32_t *meta;
-    const uint32_t *ent;                 // the lists, for atoms with too many sums for their slot
+    const uint32_t *ent;                 // the lists, for atoms coded from them
     uint32_t band_start[9];
     const uint32_t *len;
     const uint32_t *sums;                // null: code every atom from its list
@@ -109,6 +111,9 @@ void launch_fwd(const FwdJob &J, int num_sms, cudaStream_t s);
 // atoms that are all LOD0 with kept coefficients: quantise and compact only
 void launch_quant_cached(const FwdJob &J, int num_sms, cudaStream_t s);
 void launch_rc_encode(const RcJob &J, int num_sms, cudaStream_t s);
+// after launch_rc_encode with sums: the atoms that it has marked kMetaLong, their
+// lengths, and their bytes in their slots (before J.longs is used again)
+void launch_rc_long(const RcJob &J, int num_sms, cudaStream_t s);
 struct EncTables;
 void enc_tables(EncTables *t, const vcd_tables *vt);   // on the host
 // atoms that a pass for lengths takes as sets, or at once four a CTA, at most
@@ -118,6 +123,7 @@ uint64_t enc_group_atoms(int num_sms);
 void launch_resolve(const ResolveJob &J, int num_sms, cudaStream_t s);
 void launch_consume(const PlaceJob &J, cudaStream_t s);
 void launch_slots(const PlaceJob &J, cudaStream_t s);
-void launch_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, cudaStream_t s);
+// *zero: a word set to 0
+void launch_gather_dc(const uint32_t *meta, uint64_t n, uint8_t *dc, uint32_t *zero, cudaStream_t s);
 
 }  // namespace vcg

@@ -18,8 +18,8 @@ namespace vcg {
 
 // Words of an atom's slot of sums. Coders check their count every step or pair of
 // rounds (at most 256 decisions of at most 7.05 bits) and at kSumsMax or more go
-// on counting over the slot's last words; such an atom is written by
-// k_rc_encode_rest instead.
+// on counting over the slot's last words; such an atom is coded by
+// k_rc_encode_long instead.
 constexpr uint32_t kSums = 32768;
 constexpr uint32_t kSumsMax = kSums - 512;
 

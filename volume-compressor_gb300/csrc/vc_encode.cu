@@ -132,9 +132,9 @@ static void fwd_chunk(EncState &S, uint64_t c0, uint64_t n, cudaStream_t st, uin
     }
 }
 
-// coder pass over the lists of canonical atoms [c0, c0 + n)
-static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaStream_t st, uint32_t *ent,
-                       uint32_t *meta, uint32_t *sums) {
+// coder pass over the lists of canonical atoms [c0, c0 + n); of the long ones too, with `longs`
+static RcJob code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaStream_t st, uint32_t *ent,
+                        uint32_t *meta, uint32_t *sums, bool longs = true) {
     RcJob R;
     memset(&R, 0, sizeof R);
     R.n_atoms = n;
@@ -152,11 +152,13 @@ static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaS
     } else {
         // without room for sums the payloads are coded from the lists (kWrite)
         R.sums = pass == kCode ? sums + c0 * kSums : sums;
-        launch_gather_dc(meta, n, S.dc + c0, st);
+        R.longs = meta == S.meta ? S.doubt : S.doubt2;
+        launch_gather_dc(meta, n, S.dc + c0, R.longs, st);
     }
     const bool prof = vcd_prof_on();
     if (prof) cudaEventRecord(S.c->ev[5], st);
     if (pass == kSizes || R.sums) launch_rc_encode(R, g_dev.num_sms, st);
+    if (longs && R.sums) launch_rc_long(R, g_dev.num_sms, st);
     if (prof) {
         cudaEventRecord(S.c->ev[1], st);
         cudaEventSynchronize(S.c->ev[1]);
@@ -164,6 +166,7 @@ static void code_chunk(EncState &S, uint64_t c0, uint64_t n, EncPass pass, cudaS
                      0, n);
     }
     if (pass == kWrite) resolve_range(S, c0, n, ent, meta, R.sums, st);
+    return R;
 }
 
 static void run_range(EncState &S, uint64_t a0, uint64_t a1, EncPass pass, cudaStream_t st, uint32_t *ent,
@@ -193,7 +196,12 @@ static void run_split(EncState &S, uint64_t na0, uint64_t total, uint64_t chunk,
     }
     const bool first = total - na0 <= kChunk && na0 <= kChunk;
     const bool alone = first && na0 > enc_group_atoms(g_dev.num_sms);
-    cudaStream_t side = alone || vcd_prof_on() ? NULL : vcd_side_stream(c), st1 = side ? side : c->stream;
+    cudaStream_t side = vcd_prof_on() ? NULL : vcd_side_stream(c), st1 = side && !alone ? side : c->stream;
+    auto fork = [&]() {   // the side stream goes on after the work queued so far
+        if (!side) return;
+        cudaEventRecord(c->chunk_ev[0], c->stream);
+        cudaStreamWaitEvent(side, c->chunk_ev[0], 0);
+    };
     // A forward CTA takes nearly all shared memory of an SM, so beside a coder it
     // waits for the coder's CTAs: where one chunk holds each range, both forward
     // passes go first and only the coders run side by side.
@@ -201,13 +209,16 @@ static void run_split(EncState &S, uint64_t na0, uint64_t total, uint64_t chunk,
         fwd_chunk(S, na0, total - na0, c->stream, S.ent2, S.meta2);
         fwd_chunk(S, 0, na0, c->stream, S.ent, S.meta);
     }
-    if (side) {
-        cudaEventRecord(c->chunk_ev[0], c->stream);   // the side stream starts after the work queued so far
-        cudaStreamWaitEvent(side, c->chunk_ev[0], 0);
-    }
+    if (!alone) fork();
     if (first) {
-        code_chunk(S, na0, total - na0, pass, st1, S.ent2, S.meta2, sums2);
-        code_chunk(S, 0, na0, pass, c->stream, S.ent, S.meta, S.sums);
+        const bool late = pass == kCode && alone;   // the long atoms of both then go side by side, after the coders
+        const RcJob R1 = code_chunk(S, na0, total - na0, pass, st1, S.ent2, S.meta2, sums2, !late);
+        const RcJob R0 = code_chunk(S, 0, na0, pass, c->stream, S.ent, S.meta, S.sums, !late);
+        if (late) {
+            fork();
+            launch_rc_long(R1, g_dev.num_sms, side ? side : c->stream);
+            launch_rc_long(R0, g_dev.num_sms, c->stream);
+        }
     } else {
         run_range(S, na0, total, pass, st1, S.ent2, S.meta2, sums2);
         run_range(S, 0, na0, pass, c->stream, S.ent, S.meta, S.sums);
@@ -618,7 +629,10 @@ extern "C" int vcd_encode_segments(const vcd_seg *segs, int nseg, const float *q
             memcpy(R.band_start, g_dev.band_start, sizeof R.band_start);
             R.len = dlen;
             R.sums = (uint32_t *)p;
+            R.longs = drest;
+            if ((e = cudaMemsetAsync(drest, 0, 4, st)) != cudaSuccess) break;
             launch_rc_encode(R, g_dev.num_sms, st);
+            launch_rc_long(R, g_dev.num_sms, st);
             if ((e = cudaMemcpyAsync(S.len + c0, dlen, n * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
                 (e = cudaStreamSynchronize(st)) != cudaSuccess)
                 break;
