@@ -477,6 +477,28 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
 
     // ---- archive: zeroed, payloads + slots on the device, head on the host
     e = vcd_scratch(c, VCD_BUF_ARC, total + 16, &p);
+    // no room: what is held for speed alone goes first, the kept transform, then the
+    // sums and the coarser LODs' lists (the payloads are then coded from lists made
+    // anew, a chunk at a time)
+    auto give_back = [&](int slot) {
+        cudaStreamSynchronize(st);
+        cudaFree(c->buf[slot]);
+        c->buf[slot] = NULL;
+        c->cap[slot] = 0;
+    };
+    if (e == cudaErrorMemoryAllocation && S.coef) {
+        give_back(VCD_BUF_COEF);
+        S.coef = S.coef_dc = NULL;
+        S.coef_n = 0;
+        S.coef_valid = false;
+        e = vcd_scratch(c, VCD_BUF_ARC, total + 16, &p);
+    }
+    if (e == cudaErrorMemoryAllocation && (S.sums || S.ent2)) {
+        for (int slot : {(int)VCD_BUF_ESUM, (int)VCD_BUF_EENT2, (int)VCD_BUF_EMETA2}) give_back(slot);
+        S.sums = S.ent2 = S.meta2 = S.doubt2 = NULL;
+        S.whole = false;
+        e = vcd_scratch(c, VCD_BUF_ARC, total + 16, &p);
+    }
     if (e != cudaSuccess) { free(pos_h); vcd_set_error("archive buffer", e); return vcd_status_of(e); }
     S.arc = (uint8_t *)p;
     P.arc = S.arc;
