@@ -8,10 +8,13 @@
 //
 // Input (little-endian): u32 n; per stream: u32 len, u32 bad, u32 nent, then
 // len stream bytes, then nent entries (scan position | level << 16, scan order).
+// With a second argument, that many bytes are claimed past each stream, of which
+// the first 2 MiB are there, and zero: more than an atom takes.
 // Output: one line per form of the loop, "<name> <streams that differ> <streams
 // without an end> <streams with a load outside> <streams>".
 #include <stdint.h>
 #include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 #include <vector>
 
@@ -88,14 +91,14 @@ struct Result {
 };
 
 template <int kZ>
-static Result decode(const uint8_t *src, uint32_t len, const uint32_t *bs) {
+static Result decode(const uint8_t *src, uint32_t len, size_t there, const uint32_t *bs) {
     const uint32_t cap = 32768;   // VCD_MAX_ENTRIES
     std::vector<uint32_t> dst(cap);
     uint32_t S[12];
     RcLane L;
     g_votes = g_outside = 0;
     g_lo = src;
-    g_hi = src + len;
+    g_hi = src + there;
     bool ended = true;
     try {
         L.init(src, len, true, bs, S, 1, dst.data(), cap);
@@ -113,6 +116,8 @@ int main(int argc, char **argv) {
     if (argc < 2) return 2;
     FILE *f = fopen(argv[1], "rb");
     if (!f) return 2;
+    const uint32_t more = argc > 2 ? (uint32_t)strtoul(argv[2], nullptr, 0) : 0u;
+    const size_t pad = more ? 2u << 20 : 0u;
     uint32_t n = 0;
     if (fread(&n, 4, 1, f) != 1) return 2;
     uint32_t bs[10];   // the band table and a copy of its end, as the kernels hold it
@@ -129,12 +134,13 @@ int main(int argc, char **argv) {
         std::vector<uint32_t> want(nent);
         if (nent && fread(want.data(), 4, nent, f) != nent) return 2;
         // whole words that hold a stream byte, and nothing after them
-        const size_t words = (mis + len + 3u) / 4u;
+        const size_t words = (mis + len + pad + 3u) / 4u;
         uint32_t *buf = new uint32_t[words ? words : 1];
         memset(buf, 0xA5, 4 * (words ? words : 1));
         uint8_t *src = reinterpret_cast<uint8_t *>(buf) + mis;
         if (len) memcpy(src, in.data(), len);
-        const Result r[2] = {decode<0>(src, len, bs), decode<6>(src, len, bs)};
+        memset(src + len, 0, pad);
+        const Result r[2] = {decode<0>(src, len + more, len + pad, bs), decode<6>(src, len + more, len + pad, bs)};
         for (int d = 0; d < 2; ++d) {
             endless[d] += !r[d].ended;
             outside[d] += r[d].outside != 0;

@@ -84,7 +84,7 @@ def overlong_streams():
     return out
 
 
-def run(harness, oracle, streams, tmp_path):
+def run(harness, oracle, streams, tmp_path, *more):
     path = str(tmp_path / "streams.bin")
     with open(path, "wb") as f:
         f.write(struct.pack("<I", len(streams)))
@@ -93,7 +93,7 @@ def run(harness, oracle, streams, tmp_path):
             f.write(struct.pack("<III", len(s), bad, len(ent)))
             f.write(s)
             f.write(ent.astype("<u4").tobytes())
-    r = subprocess.run([harness, path], capture_output=True, text=True, timeout=900)
+    r = subprocess.run([harness, path, *more], capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stderr[-3000:]
     return {name: (int(diff), int(endless), int(outside)) for name, diff, endless, outside, _ in
             (line.split() for line in r.stdout.strip().splitlines())}
@@ -108,3 +108,9 @@ def test_overlong_prefix_ends(harness, oracle, tmp_path):
 
 def test_noise_cut_and_random_streams(harness, oracle, tmp_path):
     assert run(harness, oracle, other_streams(oracle), tmp_path) == {"dense": (0, 0, 0), "zeros": (0, 0, 0)}
+
+
+@pytest.mark.parametrize("more", ["0x7FFFFFFF", "0x80000064", "0xFFF00000"])
+def test_length_past_two_gigabytes(harness, oracle, tmp_path, more):
+    """A payload may claim up to 4 GiB; the decoder takes what its levels need."""
+    assert run(harness, oracle, other_streams(oracle), tmp_path, more) == {"dense": (0, 0, 0), "zeros": (0, 0, 0)}

@@ -313,6 +313,10 @@ constexpr uint32_t kLaneDone = 15u;
 constexpr uint32_t kLaneRows = 17u;          // shared-memory rows of a warp: 13 contexts, and rows only prefetched
 constexpr uint32_t kLaneRow = 128u;          // bytes of a row: a word per lane
 constexpr int kEscBits = 4;                  // escape bits a round takes
+// Stream bytes from which on more make no difference, and whose distances fit 31
+// bits: an atom takes less than 2 MiB (32,768 positions of 13 decisions of at most
+// 8 bits, an escape of 65 and a sign).
+constexpr uint32_t kLaneMaxLen = 1u << 30;
 constexpr uint32_t kLaneSel = 0x2107u;       // permute selector: code << 8 | first byte of the window
 
 #ifdef __CUDA_ARCH__
@@ -402,7 +406,7 @@ struct RcLane {
     // step c); host: 12 words st apart
     __device__ __forceinline__ void init(const uint8_t *s, uint32_t l, bool active, const uint32_t *bstart,
                                          uint32_t *S, uint32_t st, uint32_t *d, uint32_t cp) {
-        const uint32_t len = active ? l : 0u;
+        const uint32_t len = !active ? 0u : l < kLaneMaxLen ? l : kLaneMaxLen;
         end = s + len;
         uint32_t cd = 0, at = 5;
 #pragma unroll
