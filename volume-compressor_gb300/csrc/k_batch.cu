@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kRcBatchThreads) k_rc_batch(BatchJob J) {
         if (staged) {
             __syncwarp();   // lane 0 is done with the slice (its previous atom)
             const uint32_t len = active ? e.len - 1u : 0u;
-            in_smem = active && len + kStagePad <= kBatchStage;
+            in_smem = active && stage_fits(len, kBatchStage);
             if (in_smem) stage_stream(stage, J.arc + e.off + 1, len, lane);
             __syncwarp();
             if (lane != 0) continue;

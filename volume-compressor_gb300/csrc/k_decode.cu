@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(32) k_rc_decode(DecodeJob J, uint32_t G, uint3
     bool in_smem = false;
     if (staged) {
         const uint32_t len = active ? e.len - 1u : 0u;
-        in_smem = active && len + kStagePad <= stage_bytes;
+        in_smem = active && stage_fits(len, stage_bytes);
         if (in_smem) {
             stage_stream(stage, J.arc + e.off + 1, len, lane);
             __syncwarp();
@@ -338,8 +338,7 @@ static uint32_t stage_bytes_for(uint64_t n, uint32_t max_len, uint32_t sms) {
     const uint64_t per_sm = (n + sms - 1) / sms;
     const uint64_t room = 228ull * 1024u / per_sm;
     const uint32_t fit = room > 1280u ? (uint32_t)(room - 1152u < kStageMax ? room - 1152u : kStageMax) & ~127u : 0u;
-    const uint32_t need = (max_len + kStagePad + 127u) & ~127u;
-    if (need <= fit) return need;
+    if (stage_fits(max_len, fit)) return (max_len + kStagePad + 127u) & ~127u;
     return n <= 4ull * sms ? fit : 0u;
 }
 

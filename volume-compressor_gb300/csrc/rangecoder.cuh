@@ -796,6 +796,10 @@ __device__ __forceinline__ int rc_decode_levels_lat(const uint8_t *src, uint32_t
 constexpr uint32_t kRunZeros = 4;
 constexpr uint32_t kRunProb = 2560;     // of 4096
 constexpr uint32_t kStagePad = 16;      // zero bytes staged after a stream
+// whether a stream and those fit in room bytes (of a length near 2^32 their sum wraps)
+__host__ __device__ __forceinline__ bool stage_fits(uint32_t len, uint32_t room) {
+    return room >= kStagePad && len <= room - kStagePad;
+}
 
 // byte i of a staged stream (words are kept most significant byte first)
 __device__ __forceinline__ uint32_t stage_at(uint32_t i) { return i ^ 3u; }

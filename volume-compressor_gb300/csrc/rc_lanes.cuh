@@ -48,7 +48,7 @@ template <class Sink>
 __device__ __forceinline__ int solo_decode(uint8_t *stage, const uint8_t *src, uint32_t len, const uint32_t *bstart,
                                            Sink &&sink) {
     const uint32_t lane = threadIdx.x & 31u;
-    const bool fits = len + kStagePad <= kSoloStage;
+    const bool fits = stage_fits(len, kSoloStage);
     if (fits) stage_stream(stage, src, len, lane);
     __syncwarp();
     if (lane) return 0;
