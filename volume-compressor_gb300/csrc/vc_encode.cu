@@ -282,9 +282,13 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     const uint64_t na0 = S.lay.base[1];
     const uint64_t chunk = total_atoms < kChunk ? total_atoms : kChunk;
     // a rate control of few atoms takes three quantisers at once
-    const bool three = !info->fixed_q && 3 * na0 <= size_sets_atoms(g_dev.num_sms);
-    const uint64_t lists = three && 3 * na0 > chunk ? 3 * na0 : chunk;
+    bool three = !info->fixed_q && 3 * na0 <= size_sets_atoms(g_dev.num_sms);
+    uint64_t lists = three && 3 * na0 > chunk ? 3 * na0 : chunk;
     S.sets = 1;
+    if (lists > chunk && vcd_scratch(c, VCD_BUF_EENT, lists * VCD_MAX_ENTRIES * 4 + 16, &p) != cudaSuccess) {
+        three = false;   // no room: one at a time
+        lists = chunk;
+    }
     CK(vcd_scratch(c, VCD_BUF_EENT, lists * VCD_MAX_ENTRIES * 4 + 16, &p), "coefficient lists");
     S.ent = (uint32_t *)p;
     // quant table (8 LODs) | meta (lists) | doubt (1 + lists) | len (all atoms or lists) | dc (all atoms)
@@ -478,8 +482,8 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     // ---- archive: zeroed, payloads + slots on the device, head on the host
     e = vcd_scratch(c, VCD_BUF_ARC, total + 16, &p);
     // no room: what is held for speed alone goes first, the kept transform, then the
-    // sums and the coarser LODs' lists (the payloads are then coded from lists made
-    // anew, a chunk at a time)
+    // sums, the coarser LODs' lists and those of more than a chunk (the payloads are
+    // then coded from lists made anew, a chunk at a time)
     auto give_back = [&](int slot) {
         cudaStreamSynchronize(st);
         cudaFree(c->buf[slot]);
@@ -493,11 +497,15 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
         S.coef_valid = false;
         e = vcd_scratch(c, VCD_BUF_ARC, total + 16, &p);
     }
-    if (e == cudaErrorMemoryAllocation && (S.sums || S.ent2)) {
+    if (e == cudaErrorMemoryAllocation && (S.sums || S.ent2 || lists > chunk)) {
         for (int slot : {(int)VCD_BUF_ESUM, (int)VCD_BUF_EENT2, (int)VCD_BUF_EMETA2}) give_back(slot);
         S.sums = S.ent2 = S.meta2 = S.doubt2 = NULL;
         S.whole = false;
+        if (lists > chunk) give_back(VCD_BUF_EENT);
         e = vcd_scratch(c, VCD_BUF_ARC, total + 16, &p);
+        void *pe = S.ent;
+        if (e == cudaSuccess) e = vcd_scratch(c, VCD_BUF_EENT, chunk * VCD_MAX_ENTRIES * 4 + 16, &pe);
+        S.ent = (uint32_t *)pe;
     }
     if (e != cudaSuccess) { free(pos_h); vcd_set_error("archive buffer", e); return vcd_status_of(e); }
     S.arc = (uint8_t *)p;
