@@ -200,7 +200,6 @@ struct MmaAtom {
     uint32_t n;                // its entries
     uint32_t tensor;           // 1: a list for the tensor cores; 0: the caller's other way
     int32_t dc;
-    uint32_t lod;
     uint64_t id;               // the caller's
     Crop crop;                 // where its voxels go (plain decode)
     uint8_t *out;
@@ -221,7 +220,7 @@ struct MmaShared {
     uint32_t gave_up;          // a wait of the 16 warps ran out: set before an arrival at scattered, read after them all
     uint32_t starved;          // a wait of the feeders did
     FeedExtent<kMmaFeeders / 32> extent;
-    int2 dq[VCD_NCLASS];       // step, bias + 128 of the feeders' LOD
+    int2 dq[VCD_NCLASS];       // step, bias + 128
 };
 constexpr uint32_t kMmaLast = 1u << 30;
 
@@ -277,8 +276,7 @@ __device__ __forceinline__ void mma_release(MmaShared &M) {
 
 // The feeding warps: describe(i, a) gives atom i of the CTA or returns false
 // after the last one (called by one warp, 32 atoms at once, so that their table
-// entries, counts and offsets load together); dq: the LODs' tables; place: see
-// vcd_tables.
+// entries, counts and offsets load together); place: see vcd_tables.
 // A thread whose wait for a free chunk ran out writes no chunk any more but meets
 // the others at every barrier, until they all return before the next 32 atoms.
 template <class Describe>
@@ -288,18 +286,18 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
     constexpr int kB = kMmaChunk / kMmaFeeders;   // a chunk's list loads, then its lookups, in flight together
     uint32_t c = 0;        // chunks handed over
     bool ok = true;
-    int lod = -1;
     uint32_t w[kB];        // the list of the chunk in hand: loaded while the one before is worked on
     auto load = [&](const uint32_t *src, uint32_t m) {
 #pragma unroll
         for (int j = 0; j < kB; ++j) w[j] = (uint32_t)(j * kMmaFeeders + tid) < m ? __ldg(src + j * kMmaFeeders + tid) : 0u;
     };
     auto entries = [&](const MmaAtom &a) { return a.more && a.tensor ? a.n : 0u; };
+    for (int k = tid; k < VCD_NCLASS; k += kMmaFeeders) M.dq[k] = make_int2(dq->step[k], dq->bias[k] + 128);
     for (uint32_t i = 0;; ++i) {
         if (i % 32u == 0) {
             if (warp == 0) {
                 MmaAtom a;
-                a.n = a.tensor = a.lod = 0;
+                a.n = a.tensor = 0;
                 a.more = describe(i + lane, a);
                 M.atom[(i + lane) % kMmaAtoms] = a;
             }
@@ -310,12 +308,6 @@ __device__ __forceinline__ void mma_feed(MmaShared &M, uint8_t *ring, const vcd_
         const uint32_t n = entries(a);
         const uint32_t *src = a.src;
         if (i % 32u == 0) load(src, n);   // (else loaded with the atom before)
-        if (n && (int)a.lod != lod) {
-            lod = (int)a.lod;
-            mma_sync_feeders();
-            for (int k = tid; k < VCD_NCLASS; k += kMmaFeeders) M.dq[k] = make_int2(dq[lod].step[k], dq[lod].bias[k] + 128);
-            mma_sync_feeders();
-        }
         float norm = 0.0f;
         uint32_t far = 0;
         for (uint32_t i0 = 0;; i0 += kMmaChunk) {

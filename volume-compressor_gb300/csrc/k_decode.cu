@@ -470,7 +470,6 @@ __global__ void __launch_bounds__(kMmaCta, 1) k_idct(DecodeJob J) {
             box_atom(J, t, az, ay, ax);
             const vcd_atom e = J.atoms[job_atom(J, t, az, ay, ax)];
             a.id = t;
-            a.lod = 0;
             a.src = J.ent + J.ent_off[t];
             const uint32_t c = e.kind == VCD_PRESENT ? J.cnt[t] : kEntBad;
             a.n = c & kEntMask;
@@ -510,7 +509,7 @@ void launch_idct(const DecodeJob &J, int num_sms, cudaStream_t s, uint64_t t_lo,
     Jr.t_hi = t_hi;
     const uint64_t n = t_hi - t_lo;
     const uint64_t grid = n < (uint64_t)num_sms ? n : (uint64_t)num_sms;
-    if (n < kMmaAtomsPerSm * (uint64_t)num_sms) {
+    if (!J.place || n < kMmaAtomsPerSm * (uint64_t)num_sms) {   // (the no-alloc path: at most 64 atoms, no places)
         smem_attr((const void *)k_idct_bf, (int)kIdctTileBytes);
         k_idct_bf<<<(unsigned)grid, kBfThreads, kIdctTileBytes, s>>>(Jr);
     } else {
@@ -535,12 +534,6 @@ void launch_decode_front(const DecodeJob &J, int num_sms, cudaStream_t s, const 
     if (ev) cudaEventRecord(ev->ev[1], s);
     if (J.n_atoms) launch_rc(J, num_sms, s, ev);
     if (ev) cudaEventRecord(ev->ev[2], s);
-}
-
-void launch_decode(const DecodeJob &J, int num_sms, cudaStream_t s, const StageEvents *ev) {
-    launch_decode_front(J, num_sms, s, ev);
-    launch_idct(J, num_sms, s, 0, J.n_atoms);
-    if (ev) cudaEventRecord(ev->ev[3], s);
 }
 
 }  // namespace vcg

@@ -21,13 +21,13 @@ struct DecodeJob {
     uint32_t x0, y0, z0, x1, y1, z1;   // box
     uint8_t *out;                // box raster (x fastest)
     uint64_t ox, oy;             // box extent x, y
-    uint32_t *ent;               // coefficient lists: raster index | level << 16
+    uint32_t *ent;               // coefficient lists: scan position | level << 16
     uint64_t *ent_off;           // per box atom: first list slot (after the scan)
     uint32_t *cnt;               // per box atom: entries | flags
     const vcd_dq *dq;            // dequant tables of the LOD
     const uint32_t *alt_mask;    // step-class alternate bits
     const uint16_t *scan;        // scan position -> raster
-    const uint32_t *place;       // scan position -> place and step class (vcd_tables)
+    const uint32_t *place;       // scan position -> place and step class (vcd_tables); null: k_idct_bf alone
     uint32_t *err;               // lowest malformed box atom (atomicMin)
     uint32_t *fail;              // set when a kernel gave up a wait (zero before)
     unsigned long long *nnz_total;   // coefficient-list entries written (sum over atoms)
@@ -88,7 +88,6 @@ struct BatchJob {
     const vcd_dq *dq;            // per LOD
     const uint32_t *alt_mask;
     const uint16_t *scan;
-    const uint32_t *place;
     uint32_t *work;              // transform work counter (reset per batch)
     uint32_t *req_err;           // per request: set when one of its atoms is malformed
     uint32_t band_start[9];
@@ -141,7 +140,6 @@ inline uint32_t rc_solo_for(uint64_t n_atoms, uint32_t sms) {
 void launch_batch(const BatchJob &J, const BatchShape &shape, int num_sms, uint32_t max_ua, cudaStream_t s,
                   cudaEvent_t mid = nullptr);
 
-void launch_decode(const DecodeJob &J, int num_sms, cudaStream_t s, const StageEvents *ev);
 // The decode in two halves: list placement + range decode (events ev[0..2]),
 // then the inverse transform of box atoms [t_lo, t_hi).
 void launch_decode_front(const DecodeJob &J, int num_sms, cudaStream_t s, const StageEvents *ev);

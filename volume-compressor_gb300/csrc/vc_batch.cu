@@ -136,7 +136,6 @@ extern "C" int vcd_decode_batch(vcd_archive *d, const vcd_batch *b, uint8_t *con
     J.dq = d->dq;
     J.alt_mask = g_dev.tables->alt_mask;
     J.scan = g_dev.tables->scan;
-    J.place = g_dev.tables->place;
     J.work = ctl + 1;
     J.req_err = ctl + 4;
     memcpy(J.band_start, g_dev.band_start, sizeof J.band_start);

@@ -32,8 +32,7 @@ constexpr size_t kNaAtoms = kNaCtl + 256;                                  // 64
 constexpr size_t kNaDq = kNaAtoms + NA_MAX_ATOMS * sizeof(vcd_atom);       // vcd_dq
 constexpr size_t kNaScan = kNaDq + ((sizeof(vcd_dq) + 255) / 256) * 256;   // scan order: 32768 x u16
 constexpr size_t kNaAlt = kNaScan + 32768 * 2;                             // step-class bits: 1024 x u32
-constexpr size_t kNaPlace = kNaAlt + 4096;                                 // places and step classes: 32768 x u32
-constexpr size_t kNaBytes = kNaPlace + 32768 * 4;                          // ~8.2 MiB
+constexpr size_t kNaBytes = kNaAlt + 4096;                                 // ~8.07 MiB
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
@@ -61,7 +60,6 @@ static int na_setup(int dev, uint8_t **base, int *sms) {
             uint8_t *b = (uint8_t *)p;
             e = cudaMemcpy(b + kNaScan, t.scan, sizeof t.scan, cudaMemcpyHostToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(b + kNaAlt, t.alt_mask, sizeof t.alt_mask, cudaMemcpyHostToDevice);
-            if (e == cudaSuccess) e = cudaMemcpy(b + kNaPlace, t.place, sizeof t.place, cudaMemcpyHostToDevice);
             if (e == cudaSuccess) e = cudaMemcpy(b + kNaOff, offs, sizeof offs, cudaMemcpyHostToDevice);
         }
         if (e != cudaSuccess) {
@@ -146,7 +144,6 @@ VC_API int vcg_decode_atoms_noalloc(const uint8_t *payload_dev, size_t payload_b
     J.dq = reinterpret_cast<const vcd_dq *>(base + kNaDq);
     J.alt_mask = reinterpret_cast<const uint32_t *>(base + kNaAlt);
     J.scan = reinterpret_cast<const uint16_t *>(base + kNaScan);
-    J.place = reinterpret_cast<const uint32_t *>(base + kNaPlace);
     J.err = reinterpret_cast<uint32_t *>(base + kNaCtl);
     J.fail = J.err + 1;
     J.nnz_total = reinterpret_cast<unsigned long long *>(base + kNaCtl + 8);
