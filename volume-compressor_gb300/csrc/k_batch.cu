@@ -15,7 +15,7 @@
 
 namespace vcg {
 
-constexpr size_t kTileSmem = kIdctTileBytes;   // the butterfly's padded tile + its row lists (idct_tile.cuh)
+constexpr size_t kTileSmem = kIdctTileBytes;   // the butterfly's padded tile (idct_tile.cuh)
 
 // Persistent over the batch's distinct atoms (their number is read from device
 // memory) while the policy keeps one atom per warp (rc_lanes_for gives 1):

@@ -109,10 +109,6 @@ __device__ __forceinline__ int32_t inv_centre(const DctJob &J, uint64_t a) {
 }
 
 // ------------------------------------------------------------------ butterfly
-// One atom through the three passes with T as the padded 32 slabs x 32x32 i32
-// tile of dct32.cuh: x and y per slab (warp per
-// slab, lane per line), then z per column (thread per column) straight to the
-// output. Starts and ends with the CTA converged.
 // Whole rows (z, y) = tid + NT k of atom a.
 template <int NT>
 __device__ __forceinline__ void whole_rows(const DctJob &J, uint64_t a, uint4 (&w)[2048 / NT]) {
@@ -127,7 +123,11 @@ __device__ __forceinline__ void whole_rows(const DctJob &J, uint64_t a, uint4 (&
     }
 }
 
-// w: atom a's rows (whole_rows) for the forward, replaced by atom next's.
+// One atom through the three passes with T as the padded 32 slabs x 32x32 i32
+// tile of dct32.cuh: x (forward: a thread's rows, from its registers) and y per
+// slab (warp per slab, lane per line), then z per column (thread per column)
+// straight to the output. Starts and ends with the CTA converged. w: atom a's
+// rows (whole_rows) for the forward, replaced by atom next's.
 template <bool INV, int NT>
 __device__ void bf_atom(int32_t *T, const DctJob &J, uint64_t a, uint64_t next, uint4 (&w)[2048 / NT]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

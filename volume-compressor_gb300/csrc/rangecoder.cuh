@@ -305,10 +305,11 @@ __device__ __forceinline__ int rc_decode_levels_warp(const uint8_t *src, uint32_
 // * What a lane may meet near the end of its stream or of a band (bytes past
 //   the end read as zero, a fresh significance context, the EOB) is left to a
 //   second form of the round (END), taken when a lane of the warp is near one.
-// Measured (1,024 atoms of the 1024^3 benchmark volume, replicated to 32,768
-// in warps of 32 different ones; before: one decision a step, whatever its
-// kind, 82 instructions): 8.62 -> 4.4 ms at target 10 (kZ = 0), 6.15 -> 2.85 at
-// 20 and 1.30 -> 0.56 at 100 (kZ = 6), with the warps placed as in rc_lanes.cuh.
+// Measured on the 32,768 atoms of the 1024^3 benchmark volume, with the warps
+// placed as in rc_lanes.cuh: 5.57 ms at target 10, 3.55 at 20, 0.65 at 100. Before
+// (one decision a step, whatever its kind, 82 instructions) 8.2 ms at target 10;
+// at 20 and 100 the two were set side by side only on 1,024 of the atoms,
+// replicated: 6.15 -> 2.85 and 1.30 -> 0.56.
 constexpr uint32_t kLaneDone = 15u;
 constexpr uint32_t kLaneRows = 17u;          // shared-memory rows of a warp: 13 contexts, and rows only prefetched
 constexpr uint32_t kLaneRow = 128u;          // bytes of a row: a word per lane
@@ -645,7 +646,8 @@ struct RcLane {
         }
         round<kZ, true, true>(bstart);
     }
-    // two rounds, or one where a lane may meet an end (whole warp)
+    // two rounds, or one where a lane may meet an end (whole warp): what
+    // tests/host_decoders.cpp steps a lane with; the kernels run rounds()
     __device__ __forceinline__ void step(const uint32_t *bstart, uint32_t *S, uint32_t st) {
         (void)S;
         (void)st;

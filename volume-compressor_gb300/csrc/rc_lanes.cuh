@@ -13,18 +13,19 @@ namespace vcg {
 // different SMs; each of the other four shares a sub-partition with one of
 // them, the shortest with the longest, so that the sub-partitions carry about
 // the same work and the longest atoms, which end last, run with the shortest
-// ones or alone (warp w of a CTA runs on sub-partition w mod 4). Measured on GB300 at 32,768
-// atoms against the hardware's own placement of one-warp CTAs: 5.76 -> 5.09 ms
-// at target 10, 3.82 -> 3.34 ms at 20.
+// ones or alone (warp w of a CTA runs on sub-partition w mod 4). Measured on the
+// 32,768 atoms of the 1024^3 benchmark volume against the hardware's own placement
+// of one-warp CTAs: 5.99 -> 5.57 ms at target 10, 3.94 -> 3.55 at 20, 0.72 -> 0.65
+// at 100.
 constexpr uint32_t kLaneWarps = 8;
 constexpr int kLaneThreads = 32 * kLaneWarps;
 
 // Four more warps, one per sub-partition, take the longest atoms alone where the
 // others fill at most one warp of lanes a sub-partition: a lane's decision takes
-// two to three times as long as a lone atom's, so the longest atoms set the time,
-// and there the sub-partition has issue slots left. Beside two warps of lanes it
-// has not: 32,768 atoms take 6.40 ms with them and 5.56 without, 10,846 at target
-// 50 1.52 and 1.83, 16,969 of four LODs at target 20 5.01 and 6.73.
+// two to three times as long as a lone atom's, so the longest atoms set the time.
+// Beside two warps of lanes they slow those down by more than they save: 32,768
+// atoms take 6.40 ms with them and 5.57 without, 10,846 at target 50 1.46 and 1.83,
+// 16,969 of four LODs at target 20 4.9 and 6.73.
 constexpr uint32_t kSoloWarps = 4;
 constexpr int kLaneCta = kLaneThreads + 32 * kSoloWarps;
 constexpr uint32_t kSoloStage = 22u * 1024u;                 // stream bytes such a warp stages in shared memory
@@ -68,10 +69,13 @@ __device__ __forceinline__ uint32_t lane_warp_rank(uint32_t sms) {
 }
 
 // Payload bytes (of a warp's longest atom) from which a round takes no zeros at
-// once: longer payloads mean denser coefficients, whose runs of zeros are too
-// short to pay for it. Measured, 32,768 atoms, six zeros at once against none:
-// 4.64 against 4.50 ms at a mean of 3,220 bytes (target 10), 2.85 against
-// 3.34 ms at 1,624 (target 20), 0.56 against 0.76 ms at 323 (target 100).
+// once: longer payloads mean denser coefficients, whose runs of zeros are shorter.
+// The line comes from 1,024 atoms replicated to 32,768, six zeros at once against
+// none: 4.64 against 4.50 ms at a mean of 3,220 bytes (target 10), 2.85 against
+// 3.34 at 1,624 (target 20), 0.56 against 0.76 at 323 (target 100). The 32,768
+// different atoms of the 1024^3 benchmark volume, whose longest set the time, don't
+// bear it out: six at once for every warp 5.40, 3.19 and 0.65 ms, none 5.60, 4.13
+// and 0.91, by this line 5.57, 3.55 and 0.65.
 constexpr uint32_t kLaneDenseBytes = 2560;
 
 // The whole warp decodes its lanes' atoms (len: payload bytes, longest in lane 0).

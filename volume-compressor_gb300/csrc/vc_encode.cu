@@ -512,8 +512,8 @@ extern "C" int vcd_encode(const uint8_t *vol, int on_dev, vcd_encode_info *info,
     P.arc = S.arc;
     cudaMemsetAsync(S.arc, 0, total, st);
     if (S.whole) {
-        // (side by side: each may hold atoms coded from their lists, whose time is one
-        // atom's chain: white noise at q 0.05, 95 ms each at 640^3)
+        // (side by side: each may hold atoms past their slots, coded from their lists,
+        // whose time is one atom's chain)
         cudaStream_t side = S.ent2 && !prof ? vcd_side_stream(c) : NULL;
         if (side) {
             cudaEventRecord(c->chunk_ev[0], st);
