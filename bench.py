@@ -195,10 +195,10 @@ class Clocks:
 # What bounds each decode stage, from the ncu captures of this workload (an HBM
 # fraction alone misreads a latency-bound kernel).
 LIMITER = {
-    "rc_decode": "dependency chain of the per-lane range decoder's rounds and the issue slots of two warps per "
-                 "sub-partition: 742 MB of DRAM traffic in 5.6 ms (ncu)",
+    "rc_decode": "dependency chain of the per-lane range decoder's rounds, at most two warps per sub-partition: ALU "
+                 "52 %, issue 47 % busy; 742 MB of DRAM traffic in 5.6 ms (ncu)",
     "idct": "operand reads of the tensor cores from shared memory, the rounding epilogue and byte stores: tensor pipe "
-            "13 %, ALU 35 %, FMA-heavy 33 % busy; 1.65 GB of DRAM traffic in 2.5 ms (ncu)",
+            "14 %, ALU 37 %, FMA-heavy 34 % busy; 1.65 GB of DRAM traffic in 2.5 ms (ncu)",
 }
 
 
